@@ -360,7 +360,7 @@ struct vkb_ctx {
     DBuf<float4> accum, staging;        // per-render accumulators and host-output staging (all jobs of a call)
     DBuf<uint32_t> ids;                 // primary ids of the jobs that asked for them
     size_t wave_capacity = 32u << 20;   // path slots per wave (autotuned); 7.4 GB of queues when full
-    int trace_blocks_per_sm = 128;      // trace/shade grid = SMs x this (autotuned)
+    int trace_blocks_per_sm = 128;      // shade grid: at most SMs x this (autotuned)
     uint64_t launches = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::vector<cudaEvent_t> kernel_events;
@@ -774,6 +774,23 @@ struct CacheLaunch {
     uint32_t* err = nullptr;
 };
 
+// Grids of the queue kernels of a wave of `paths` path slots.  A queue holds at most one
+// entry per slot, and a block that finds none still costs its launch and, in a trace, an
+// atomic per warp on the fetch counter: 128 blocks per SM over an empty queue took 77 us
+// (closest hit), 58 us (shadow) and 50 us (shade), most of a small render.  The traces are
+// persistent (a warp takes rays until the counter runs out), so they need the resident
+// blocks and no more: 1920x1080 frames of the flock are equal at 8 and 128 blocks per SM.
+// The shade grid strides; more blocks than are resident balance its load, so it keeps the
+// context's blocks per SM where the wave has that many entries.
+struct WaveGrids {
+    int trace, shade;
+    WaveGrids(const vkb_ctx* c, uint32_t paths) {
+        const uint32_t sms = uint32_t(c->sms);
+        trace = int(std::max(1u, std::min((paths + TRACE_BLOCK - 1u) / TRACE_BLOCK, sms * VKB_TRACE_MIN_BLOCKS)));
+        shade = int(std::max(1u, std::min((paths + SHADE_BLOCK - 1u) / SHADE_BLOCK, sms * uint32_t(c->trace_blocks_per_sm))));
+    }
+};
+
 // The kernels of one wave: camera, then per bounce closest-hit trace, shade, shadow trace;
 // then the radiance-cache queries, if any; then accumulation.  Timed
 // mode records events around every closest-hit trace.
@@ -792,11 +809,12 @@ void launch_shadow(bool counted, int grid, cudaStream_t st, const PathParams& p)
 // st: the wave's stream; acc_wait / acc_done: events that order the accumulation after
 // the previous wave's and mark this one's (overlapped waves), or null.
 template <bool BATCH>
-void wave_kernels(vkb_ctx* c, const PathParams& p, uint32_t bounces, bool counted, bool timed, WaveTotals& tot,
+void wave_kernels(vkb_ctx* c, const PathParams& p, uint32_t paths, uint32_t bounces, bool counted, bool timed, WaveTotals& tot,
                   const CacheLaunch* cache = nullptr, bool ext = false, bool w8 = false, cudaStream_t st = nullptr,
                   cudaEvent_t acc_wait = nullptr, cudaEvent_t acc_done = nullptr) {
     if (!st) st = c->stream;
-    const int sms = c->sms, tgrid = sms * c->trace_blocks_per_sm, sgrid = sms * c->trace_blocks_per_sm;
+    const WaveGrids grids(c, paths);
+    const int sms = c->sms, tgrid = grids.trace, sgrid = grids.shade;
     const bool adaptive = !BATCH && p.job0.adaptive;
     if (adaptive) k_adaptive_decide<<<grid_for(p.job0.npix, 256, sms), 256, 0, st>>>(p);
     k_start_wave<<<1, 1, 0, st>>>(p.counters, adaptive ? 1u : 0u);
@@ -1029,14 +1047,15 @@ struct WaveEngine {
             uint64_t key = (uint64_t(bounces) << 1) | 1u;
             key = key * 1315423911ull + (counted ? 7u : 3u) + (ext ? 11u : 0u) + (w8 ? 17u : 0u);
             key = key * 40503ull + wave_jobs;
-            key = key * 97ull + uint64_t(c->trace_blocks_per_sm);
+            const WaveGrids grids(c, n_paths);
+            key = (key * 97ull + uint64_t(grids.trace)) * 19457ull + uint64_t(grids.shade);
             cudaGraphExec_t exec = nullptr;
             for (auto& g : captured) if (g.key == key) exec = g.exec;
             if (!exec) {
                 cudaGraph_t g;
                 VKB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
                 WaveTotals scratch;
-                wave_kernels<true>(c, p, bounces, counted, false, scratch, nullptr, ext, w8);
+                wave_kernels<true>(c, p, n_paths, bounces, counted, false, scratch, nullptr, ext, w8);
                 VKB_CUDA(cudaStreamEndCapture(st, &g));
                 VKB_CUDA(cudaGraphInstantiate(&exec, g, 0));
                 VKB_CUDA(cudaGraphDestroy(g));
@@ -1046,9 +1065,9 @@ struct WaveEngine {
             tot.launches += 3 + 4 * (bounces + 1);
             tot.trace_launches += bounces + 1;
         } else if (batch) {
-            wave_kernels<true>(c, p, bounces, counted, timed, tot, nullptr, ext, w8, st, acc_wait, acc_done);
+            wave_kernels<true>(c, p, n_paths, bounces, counted, timed, tot, nullptr, ext, w8, st, acc_wait, acc_done);
         } else {
-            wave_kernels<false>(c, p, bounces, counted, timed, tot, cache, ext, w8, st, acc_wait, acc_done);
+            wave_kernels<false>(c, p, n_paths, bounces, counted, timed, tot, cache, ext, w8, st, acc_wait, acc_done);
         }
         VKB_CUDA(cudaGetLastError());
         ++waves;
