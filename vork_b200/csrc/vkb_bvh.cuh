@@ -80,7 +80,6 @@ struct TraceStack {
     }
 };
 constexpr uint32_t TRACE_STEP_LIMIT = 1u << 16;
-constexpr int SENTINEL = 0x7fffffff;
 
 // ---------------------------------------------------------------- Morton codes (bit-exact with the CPU restatement)
 __device__ __forceinline__ uint32_t expand_bits(uint32_t v) {
@@ -116,10 +115,12 @@ struct RaySpace {
 };
 __device__ __forceinline__ float safe_rcp(float x) { return 1.f / (fabsf(x) > 1e-20f ? x : copysignf(1e-20f, x)); }
 __device__ __forceinline__ float comp(float3 v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
-__device__ __forceinline__ void make_space(RaySpace& r, float3 o, float3 d) {
-    r.o = o;
+// shear: also the triangle test's part (origin and shear), which no node visit reads.
+__device__ __forceinline__ void make_space(RaySpace& r, float3 o, float3 d, bool shear) {
     r.idir = f3(safe_rcp(d.x), safe_rcp(d.y), safe_rcp(d.z));
     r.ood = f3(o.x * r.idir.x, o.y * r.idir.y, o.z * r.idir.z);
+    if (!shear) return;
+    r.o = o;
     float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
     int kz = (ax > ay) ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);
     int kx = kz + 1 == 3 ? 0 : kz + 1;
@@ -258,15 +259,19 @@ struct SceneView {
 struct TraceCount { uint32_t nodes = 0, tris = 0, instances = 0, blas_nodes = 0; };
 
 // Traversal state of one ray: closest hit (ANY == false) or first hit (ANY == true) over
-// the two-level BVH, advanced one step (a 4-wide node, an instance entry, a BLAS leaf,
-// then a pop) at a time.  Error: overflow/step-limit exits set *err and end the ray with
-// the best hit so far.  W8: the BLASes are compressed 8-wide (the TLAS stays 4-wide).
+// the two-level BVH.  `node` says what comes next: a node to visit (>= 0), a BLAS leaf or
+// an instance (< 0, by in_blas), the end of an instance (LEAVE, as on the stack) or nothing
+// (DONE: hit/found hold the result).  visit() and special() advance the ray, each in the
+// stack's order whenever it is called, so the caller may hold specials back until several
+// lanes of the warp have one.  Error: overflow/step-limit exits set *err and end the ray
+// with the best hit so far.  W8: the BLASes are compressed 8-wide (the TLAS stays 4-wide).
 template <bool ANY, bool COUNT = false, bool W8 = false>
 struct TraceLane {
     static constexpr int CAP = W8 ? STACK_CAP8 : STACK_CAP;
+    static constexpr int LEAVE = int(0x80000000u), DONE = int(0x80000001u);   // below every leaf reference
     RaySpace rs;
     float tbest;
-    int node, sp;
+    int node = DONE, sp;
     bool found, in_blas, cull;
     const Bvh4Node* nodes;
     const Bvh8Node* nodes8;
@@ -275,18 +280,27 @@ struct TraceLane {
 
     // Returns false when there is nothing to traverse.
     __device__ __forceinline__ bool start(const SceneView& s, RayRef ray, float tmax) {
-        make_space(rs, ray.origin(), ray.dir());
-        tbest = tmax; node = 0; sp = 0; steps = 0;
+        make_space(rs, ray.origin(), ray.dir(), false);
+        tbest = tmax; sp = 0; steps = 0;
         found = false; in_blas = false; cull = false;
         nodes = s.tlas_nodes; tri_base = 0; cur_instance = 0;
-        return s.num_instances != 0;
+        const bool any = s.num_instances != 0;
+        node = any ? 0 : DONE;
+        return any;
     }
-    // One step; returns true when the ray is finished (hit/found hold the result).
-    __device__ __forceinline__ bool step(const SceneView& s, RayRef ray, uint32_t* err, TraceCount* count, TraceStack stk) {
-        if (++steps >= TRACE_STEP_LIMIT) { atomicOr(err, 2u); return true; }
-        bool respace = false;
-        float3 so, sd;
-        if (W8 && in_blas && node >= 0) {
+    __device__ __forceinline__ bool done() const { return node == DONE; }
+    __device__ __forceinline__ bool at_special() const { return node < 0 && node != DONE; }
+    __device__ __forceinline__ void fail(uint32_t* err, uint32_t bit) { atomicOr(err, bit); node = DONE; }
+    __device__ __forceinline__ void pop(TraceStack stk) {
+        if (sp == 0) { node = DONE; return; }
+        --sp;
+        node = stk.get(sp);
+    }
+    // A node (node >= 0): its nearest hit child next, the other hits pushed far to near, or
+    // a pop when it has none.
+    __device__ __forceinline__ void visit(uint32_t* err, TraceCount* count, TraceStack stk) {
+        if (++steps >= TRACE_STEP_LIMIT) { fail(err, 2u); return; }
+        if (W8 && in_blas) {
             // A compressed 8-wide BLAS node: decode the eight slots' planes on the ray's
             // grid (t = q * 2^e / d + (origin - o) / d), sort the hit slots' keys, descend
             // into the first and push the rest (farthest first).
@@ -329,14 +343,14 @@ struct TraceLane {
                 int pushes = 0;
                 #pragma unroll
                 for (int i = 1; i < 8; ++i) pushes += key[i] != 0xffffffffu ? 1 : 0;
-                if (sp + pushes > CAP) { atomicOr(err, 1u); return true; }
+                if (sp + pushes > CAP) { fail(err, 1u); return; }
                 #pragma unroll
                 for (int i = 7; i >= 1; --i)
                     if (key[i] != 0xffffffffu) { stk.put(sp, child(key[i])); ++sp; }
                 node = child(key[0]);
-                return false;
+                return;
             }
-        } else if (node >= 0) {
+        } else {
             if (COUNT) { count->nodes++; if (in_blas) count->blas_nodes++; }
             const float4* p = reinterpret_cast<const float4*>(nodes + node);
             const uint32_t sx = __float_as_uint(rs.idir.x) >> 31, sy = __float_as_uint(rs.idir.y) >> 31, sz = __float_as_uint(rs.idir.z) >> 31;
@@ -361,35 +375,24 @@ struct TraceLane {
                         if (k2 != 0xffffffffu) { stk.r[sp * TRACE_BLOCK] = slot_child(ch, k2); ++sp; }
                         stk.r[sp * TRACE_BLOCK] = slot_child(ch, k1); ++sp;
                     } else {
-                        if (sp + pushes > CAP) { atomicOr(err, 1u); return true; }
+                        if (sp + pushes > CAP) { fail(err, 1u); return; }
                         if (k3 != 0xffffffffu) { stk.put(sp, slot_child(ch, k3)); ++sp; }
                         if (k2 != 0xffffffffu) { stk.put(sp, slot_child(ch, k2)); ++sp; }
                         stk.put(sp, slot_child(ch, k1)); ++sp;
                     }
                 }
                 node = slot_child(ch, k0);
-                return false;
+                return;
             }
-        } else if (!in_blas) {
-            if (COUNT) count->instances++;
-            const TlasLeaf* lf = s.tlas_leaves + (~node);
-            float4 r0 = __ldg(&lf->w2o[0]), r1 = __ldg(&lf->w2o[1]), r2 = __ldg(&lf->w2o[2]);
-            uint4 info = __ldg(reinterpret_cast<const uint4*>(&lf->instance));
-            const float3 o = ray.origin(), d = ray.dir();
-            so = f3(r0.x * o.x + r0.y * o.y + r0.z * o.z + r0.w, r1.x * o.x + r1.y * o.y + r1.z * o.z + r1.w, r2.x * o.x + r2.y * o.y + r2.z * o.z + r2.w);
-            sd = f3(r0.x * d.x + r0.y * d.y + r0.z * d.z, r1.x * d.x + r1.y * d.y + r1.z * d.z, r2.x * d.x + r2.y * d.y + r2.z * d.z);
-            cur_instance = info.x;
-            if (W8) nodes8 = s.blas8 + info.y;
-            else nodes = s.blas_nodes + info.y;
-            tri_base = info.z;
-            cull = !ANY && (info.w & LEAF_CULL_BACKFACES);
-            if (sp >= CAP) { atomicOr(err, 1u); return true; }
-            stk.put(sp, SENTINEL);
-            ++sp;
-            in_blas = true;
-            node = 0;
-            respace = true;
-        } else {
+        }
+        pop(stk);
+    }
+    // A BLAS leaf, the end of an instance, an instance entry: whichever the ray is at, and
+    // then those that follow in this order without a node between them, so an instance left
+    // for another one sets up the ray's space once.
+    __device__ __forceinline__ void special(const SceneView& s, RayRef ray, uint32_t* err, TraceCount* count, TraceStack stk) {
+        if (in_blas && node != LEAVE) {
+            if (++steps >= TRACE_STEP_LIMIT) { fail(err, 2u); return; }
             // BLAS leaf: up to VKB_BLAS_LEAF_MAX triangles in leaf order, ~((first << 2) | (count - 1)).
             uint32_t v = uint32_t(~node), first = v >> 2, cnt = VKB_BLAS_LEAF_MAX == 1 ? 1u : (v & 3u) + 1u;
             for (uint32_t k = 0; k < cnt; ++k) {
@@ -400,29 +403,42 @@ struct TraceLane {
                 if (tri_test(rs, f3(v0.x, v0.y, v0.z), f3(v1.x, v1.y, v1.z), f3(v2.x, v2.y, v2.z), cull, tbest, t, b1, b2)) {
                     tbest = t; found = true;
                     hit.t = t; hit.u = b1; hit.v = b2; hit.tri = tri_base + first + k; hit.inst = cur_instance;
-                    if (ANY) return true;
+                    if (ANY) { node = DONE; return; }
                 }
             }
+            pop(stk);
         }
-        if (!respace) {
-            // pop; leaving an instance (its sentinel) goes back to the world ray
-            if (sp == 0) return true;
-            --sp;
-            node = stk.get(sp);
-            if (node != SENTINEL) return false;
-            while (node == SENTINEL) {
-                in_blas = false;
-                nodes = s.tlas_nodes;
-                if (sp == 0) return true;
-                --sp;
-                node = stk.get(sp);
-            }
-            so = ray.origin();
-            sd = ray.dir();
+        bool respace = false;
+        if (node == LEAVE) {
+            in_blas = false;
+            nodes = s.tlas_nodes;
+            pop(stk);
+            respace = true;
         }
-        // the one ray-space set-up of a step (instance entry or exit)
-        make_space(rs, so, sd);
-        return false;
+        if (node == DONE || (!respace && in_blas)) return;
+        float3 so = ray.origin(), sd = ray.dir();
+        if (node < 0) {
+            // Instance entry: the ray in object space.
+            if (++steps >= TRACE_STEP_LIMIT) { fail(err, 2u); return; }
+            if (COUNT) count->instances++;
+            const TlasLeaf* lf = s.tlas_leaves + (~node);
+            float4 r0 = __ldg(&lf->w2o[0]), r1 = __ldg(&lf->w2o[1]), r2 = __ldg(&lf->w2o[2]);
+            uint4 info = __ldg(reinterpret_cast<const uint4*>(&lf->instance));
+            const float3 o = so, d = sd;
+            so = f3(r0.x * o.x + r0.y * o.y + r0.z * o.z + r0.w, r1.x * o.x + r1.y * o.y + r1.z * o.z + r1.w, r2.x * o.x + r2.y * o.y + r2.z * o.z + r2.w);
+            sd = f3(r0.x * d.x + r0.y * d.y + r0.z * d.z, r1.x * d.x + r1.y * d.y + r1.z * d.z, r2.x * d.x + r2.y * d.y + r2.z * d.z);
+            cur_instance = info.x;
+            if (W8) nodes8 = s.blas8 + info.y;
+            else nodes = s.blas_nodes + info.y;
+            tri_base = info.z;
+            cull = !ANY && (info.w & LEAF_CULL_BACKFACES);
+            if (sp >= CAP) { fail(err, 1u); return; }
+            stk.put(sp, LEAVE);
+            ++sp;
+            in_blas = true;
+            node = 0;
+        }
+        make_space(rs, so, sd, in_blas);
     }
 };
 
@@ -431,7 +447,10 @@ __device__ __forceinline__ bool trace_ray(const SceneView& s, RayRef ray, float 
                                           TraceCount* count, TraceStack stk) {
     TraceLane<ANY, COUNT, W8> L;
     if (!L.start(s, ray, tmax)) return false;
-    while (!L.step(s, ray, err, count, stk)) {}
+    while (!L.done()) {
+        if (L.node >= 0) L.visit(err, count, stk);
+        if (L.at_special()) L.special(s, ray, err, count, stk);
+    }
     hit = L.hit;
     return L.found;
 }

@@ -728,13 +728,26 @@ __device__ __forceinline__ bool trace_any(const SceneView& sv, RayRef ray, float
 #ifndef VKB_TRACE_REFILL
 #define VKB_TRACE_REFILL 20
 #endif
+// A warp keeps visiting nodes while more than this many lanes are at one; then it takes
+// every waiting special step (leaf, instance entry and exit) together.
+#ifndef VKB_TRACE_NODES
+#define VKB_TRACE_NODES 12
+#endif
 static_assert(VKB_TRACE_REFILL >= 1 && VKB_TRACE_REFILL <= 31, "refill threshold in lanes");
-// Closest hits of the queued rays with lane refill: each lane carries one ray's
-// traversal state; once at most VKB_TRACE_REFILL lanes of a warp are still tracing, the
-// idle lanes take the next rays of the queue together (one atomic per warp), so a warp
-// does not run on with a few long rays while its other lanes wait (measured: a warp's
-// lanes otherwise spend ~60% of its steps idle behind its longest ray).  Refilling
-// each lane as soon as it finishes is slower: the refill code then runs on single lanes.
+static_assert(VKB_TRACE_NODES >= 0 && VKB_TRACE_NODES <= 31, "node threshold in lanes");
+// Closest hits of the queued rays.  Bound by instruction issue under divergence (issue 56%
+// of cycles, 10 of 32 lanes) behind dependent node fetches.  A ray's steps are ~85% node
+// visits; at two dozen rays a warp nearly always had one lane at a leaf, an instance entry
+// or exit and one finishing, so with one branch per step every pass paid for all four with
+// a lane or two in each (542 warp instructions per ray on the flock at 480x270).  So
+//  - the specials wait until at most VKB_TRACE_NODES lanes have a node (8 / 10 / 12 / 16 /
+//    20: 403.8 / 401.4 / 400.9 / 403.1 / 413.5 ms for the 1080p 64 spp flock frame; each
+//    ray's own order, and so every hit, is unchanged);
+//  - results are written, and new rays taken from the queue with one atomic, by all the
+//    warp's idle lanes together once at most VKB_TRACE_REFILL still trace (each lane as soon
+//    as it finishes is slower: that code then runs on single lanes).
+// 419 warp instructions per ray; the frame 483.0 -> 400.9 ms with the shadow rays done
+// the same way, 256x256 16 spp 2.72 -> 2.37 ms.
 template <bool COUNT, bool BATCH, bool W8 = false>
 __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace(PathParams p, int cur) {
     VKB_STACK_DECL_W(W8)
@@ -747,41 +760,30 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace(Pat
     uint32_t ray = NONE, job = 0;
     bool drained = false;
     for (;;) {
-        uint32_t act = __ballot_sync(0xffffffffu, ray != NONE);
-        if (!drained && uint32_t(__popc(act)) <= uint32_t(VKB_TRACE_REFILL)) {
+        uint32_t act = __ballot_sync(0xffffffffu, !L.done());
+        if (act == 0u || (!drained && uint32_t(__popc(act)) <= uint32_t(VKB_TRACE_REFILL))) {
+            if (ray != NONE && L.done()) {
+                p.hit[ray] = L.found ? make_float4(L.hit.t, L.hit.u, L.hit.v, __uint_as_float(L.hit.tri)) : make_float4(-1.f, 0.f, 0.f, __uint_as_float(0xffffffffu));
+                p.hit_inst[ray] = L.found ? L.hit.inst : 0xffffffffu;
+                ray = NONE;
+            }
+            if (drained) break;
             const uint32_t idle = ~act;
             uint32_t base = 0;
             if (lane == 0u) base = atomicAdd(&p.counters[11], uint32_t(__popc(idle)));
             base = __shfl_sync(0xffffffffu, base, 0);
             drained = base + uint32_t(__popc(idle)) >= n;
-            if (ray == NONE) {
-                const uint32_t r = base + uint32_t(__popc(idle & ((1u << lane) - 1u)));
-                if (r < n) {
-                    if (BATCH) job = job_of_slot<true>(p, __float_as_uint(p.ray_d[cur][r].w));
-                    if (L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.ray_o[cur], p.ray_d[cur], r}, p.ray_o[cur][r].w)) {
-                        ray = r;
-                    } else {
-                        p.hit[r] = make_float4(-1.f, 0.f, 0.f, __uint_as_float(0xffffffffu));
-                        p.hit_inst[r] = 0xffffffffu;
-                    }
-                }
+            const uint32_t r = base + uint32_t(__popc(idle & ((1u << lane) - 1u)));
+            if (L.done() && r < n) {
+                ray = r;
+                if (BATCH) job = job_of_slot<true>(p, __float_as_uint(p.ray_d[cur][r].w));
+                L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.ray_o[cur], p.ray_d[cur], r}, p.ray_o[cur][r].w);
             }
-            act = __ballot_sync(0xffffffffu, ray != NONE);
         }
-        if (act == 0u) {
-            if (drained) break;
-            continue;
-        }
-        bool done = false;
-        if (ray != NONE) {
-            if constexpr (BATCH) done = L.step(p.jobs[job].sv, RayRef{p.ray_o[cur], p.ray_d[cur], ray}, p.err, &tc, stk);
-            else done = L.step(p.job0.sv, RayRef{p.ray_o[cur], p.ray_d[cur], ray}, p.err, &tc, stk);
-        }
-        if (done) {
-            p.hit[ray] = L.found ? make_float4(L.hit.t, L.hit.u, L.hit.v, __uint_as_float(L.hit.tri)) : make_float4(-1.f, 0.f, 0.f, __uint_as_float(0xffffffffu));
-            p.hit_inst[ray] = L.found ? L.hit.inst : 0xffffffffu;
-            ray = NONE;
-        }
+        if (L.at_special()) L.special(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.ray_o[cur], p.ray_d[cur], ray}, p.err, &tc, stk);
+        do {
+            if (L.node >= 0) L.visit(p.err, &tc, stk);
+        } while (__popc(__ballot_sync(0xffffffffu, L.node >= 0)) > VKB_TRACE_NODES);
     }
     if (COUNT) {
         flush_count(&p.work[0], tc.nodes);
@@ -856,30 +858,31 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace_sha
     };
     bool drained = false;
     for (;;) {
-        uint32_t act = __ballot_sync(0xffffffffu, e != NONE);
-        if (!drained && uint32_t(__popc(act)) <= uint32_t(VKB_TRACE_REFILL)) {
-            const uint32_t idle = ~act;
-            uint32_t base = 0;
-            if (lane == 0u) base = atomicAdd(&p.counters[12], uint32_t(__popc(idle)));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            drained = base + uint32_t(__popc(idle)) >= n;
-            if (e == NONE) {
+        uint32_t act = __ballot_sync(0xffffffffu, !L.done());
+        if (act == 0u || (!drained && uint32_t(__popc(act)) <= uint32_t(VKB_TRACE_REFILL))) {
+            if (e != NONE && L.done()) {
+                if (L.found) occ |= 1u << phase;
+                if constexpr (EXT) { if (phase == 3u || !begin(phase + 1u)) finish(); }
+                else { if (phase != 0u || !begin(1u)) finish(); }
+            }
+            const uint32_t idle = __ballot_sync(0xffffffffu, e == NONE);
+            if (drained) {
+                if (idle == 0xffffffffu) break;
+            } else {
+                uint32_t base = 0;
+                if (lane == 0u) base = atomicAdd(&p.counters[12], uint32_t(__popc(idle)));
+                base = __shfl_sync(0xffffffffu, base, 0);
+                drained = base + uint32_t(__popc(idle)) >= n;
                 const uint32_t r = base + uint32_t(__popc(idle & ((1u << lane) - 1u)));
-                if (r < n) {
+                if (e == NONE && r < n) {
                     e = r;
                     occ = 0u;
                     if (BATCH) job = job_of_slot<true>(p, __float_as_uint(p.sa_d[r].w));
                     if (!begin(0u)) finish();
                 }
             }
-            act = __ballot_sync(0xffffffffu, e != NONE);
         }
-        if (act == 0u) {
-            if (drained) break;
-            continue;
-        }
-        bool done = false;
-        if (e != NONE) {
+        if (L.at_special()) {
             // The traversal re-reads its ray (instance entry, return to world space):
             // phase 0 the light ray A, 1 the light ray B, 2 the environment ray, 3 the mesh ray.
             RayRef ray{phase ? p.sb_o : p.sa_o, phase ? p.sb_d : p.sa_d, rid};
@@ -887,14 +890,11 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace_sha
                 if (phase == 2u) ray = RayRef{p.sc_o, p.sc_d, rid};
                 else if (phase == 3u) ray = RayRef{p.sd_o, p.sd_d, rid};
             }
-            if constexpr (BATCH) done = L.step(p.jobs[job].sv, ray, p.err, &tc, stk);
-            else done = L.step(p.job0.sv, ray, p.err, &tc, stk);
+            L.special(BATCH ? p.jobs[job].sv : p.job0.sv, ray, p.err, &tc, stk);
         }
-        if (done) {
-            if (L.found) occ |= 1u << phase;
-            if constexpr (EXT) { if (phase == 3u || !begin(phase + 1u)) finish(); }
-            else { if (phase != 0u || !begin(1u)) finish(); }
-        }
+        do {
+            if (L.node >= 0) L.visit(p.err, &tc, stk);
+        } while (__popc(__ballot_sync(0xffffffffu, L.node >= 0)) > VKB_TRACE_NODES);
     }
     if (COUNT) {
         flush_count(&p.work[3], tc.nodes);
