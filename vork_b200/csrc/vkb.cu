@@ -783,10 +783,11 @@ struct CacheLaunch {
 // The shade grid strides; more blocks than are resident balance its load, so it keeps the
 // context's blocks per SM where the wave has that many entries.
 struct WaveGrids {
-    int trace, shade;
+    int trace, split, shade;
     WaveGrids(const vkb_ctx* c, uint32_t paths) {
         const uint32_t sms = uint32_t(c->sms);
         trace = int(std::max(1u, std::min((paths + TRACE_BLOCK - 1u) / TRACE_BLOCK, sms * VKB_TRACE_MIN_BLOCKS)));
+        split = int(std::max(1u, std::min((paths + SPLIT_BLOCK - 1u) / SPLIT_BLOCK, sms * 16u)));
         shade = int(std::max(1u, std::min((paths + SHADE_BLOCK - 1u) / SHADE_BLOCK, sms * uint32_t(c->trace_blocks_per_sm))));
     }
 };
@@ -834,14 +835,15 @@ void wave_kernels(vkb_ctx* c, const PathParams& p, uint32_t paths, uint32_t boun
         if (timed) VKB_CUDA(cudaEventRecord(c->kernel_events[2 * tot.trace_launches + 1], st));
         tot.trace_launches++;
         if (!BATCH && b == 0u && p.guide) { k_guides<<<sms * 8, 256, 0, st>>>(p); tot.launches += 1; }
-        k_reset_queues<<<1, 1, 0, st>>>(p.counters, cur ^ 1);
         // Waves with an image environment or emissive meshes run the kernels with their
         // strategies (two more shadow rays per vertex); the others keep the plain ones.
         if (ext) {
+            k_split<BATCH, true><<<grids.split, SPLIT_BLOCK, 0, st>>>(p, cur);
             k_shade<BATCH, true><<<sgrid, SHADE_BLOCK, 0, st>>>(p, cur);
             if (w8) launch_shadow<BATCH, true, true>(counted, tgrid, st, p);
             else launch_shadow<BATCH, true, false>(counted, tgrid, st, p);
         } else {
+            k_split<BATCH, false><<<grids.split, SPLIT_BLOCK, 0, st>>>(p, cur);
             k_shade<BATCH, false><<<sgrid, SHADE_BLOCK, 0, st>>>(p, cur);
             if (w8) launch_shadow<BATCH, false, true>(counted, tgrid, st, p);
             else launch_shadow<BATCH, false, false>(counted, tgrid, st, p);

@@ -502,7 +502,8 @@ struct PathParams {
     float4* sb_o; float4* sb_d; float4* sb_c;
     // [0],[1] ray counts, [2] shadow count, [3] ext rays, [4] shadow rays, [5] dropped light,
     // [6] dropped paths, [7] path slots of this wave, [8] pixels of this wave's jobs
-    // [9] radiance-cache records of this wave, [10] adaptive pixel-samples skipped
+    // [9] radiance-cache records of this wave, [10] adaptive pixel-samples skipped,
+    // [11], [12] rays the closest-hit and shadow traces have taken, [13] this bounce's hits
     uint32_t* counters;
     unsigned long long* work;  // instrumented traversal: closest nodes, tris, instances, blas nodes; shadow nodes, tris, blas nodes
     uint32_t* err;
@@ -602,16 +603,6 @@ __device__ __forceinline__ float filter_offset(const float* table, float u) {
     uint32_t i = min(uint32_t(x), FILTER_INTERVALS - 1u);
     return lerpf(__ldg(table + i), __ldg(table + i + 1), x - float(i));
 }
-// Warp-aggregated queue append: one atomic per warp.
-__device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool want) {
-    uint32_t mask = __ballot_sync(0xffffffffu, want);
-    if (!want) return 0xffffffffu;
-    uint32_t lane = threadIdx.x & 31u, leader = __ffs(mask) - 1u;
-    uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(counter, __popc(mask));
-    base = __shfl_sync(mask, base, leader);
-    return base + __popc(mask & ((1u << lane) - 1u));
-}
 // Queue append by the threads of a warp that reach it together (one atomic per group).
 __device__ __forceinline__ uint32_t group_append(uint32_t* counter) {
     const uint32_t mask = __activemask(), lane = threadIdx.x & 31u, leader = __ffs(mask) - 1u;
@@ -620,33 +611,6 @@ __device__ __forceinline__ uint32_t group_append(uint32_t* counter) {
     base = __shfl_sync(mask, base, leader);
     return base + uint32_t(__popc(mask & ((1u << lane) - 1u)));
 }
-// Shade appends a new extension ray or shadow entry where it makes it (the threads of a
-// warp that get there together share one atomic) instead of carrying five float4s to a
-// warp-wide append at the end of the loop body: 128 registers with 12/16 B of spill
-// instead of 108/156 B (measured: 618 vs 623 ms per large frame).
-// The same, with the group's slots ordered by key (0..7; ties by lane): the entries a
-// trace warp later takes together then share their direction octant where they can.
-__device__ __forceinline__ uint32_t group_append_by_key(uint32_t* counter, uint32_t key) {
-    const uint32_t mask = __activemask(), lane = threadIdx.x & 31u, leader = __ffs(mask) - 1u;
-    const uint32_t k0 = __ballot_sync(mask, key & 1u), k1 = __ballot_sync(mask, key & 2u), k2 = __ballot_sync(mask, key & 4u);
-    uint32_t below = 0, same = 0;
-    #pragma unroll
-    for (uint32_t k = 0; k < 8; ++k) {
-        const uint32_t with = mask & ((k & 1u) ? k0 : ~k0) & ((k & 2u) ? k1 : ~k1) & ((k & 4u) ? k2 : ~k2);
-        if (k < key) below += uint32_t(__popc(with));
-        if (k == key) same = with;
-    }
-    uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(counter, uint32_t(__popc(mask)));
-    base = __shfl_sync(mask, base, leader);
-    return base + below + uint32_t(__popc(same & ((1u << lane) - 1u)));
-}
-#ifndef VKB_SHADE_OCTANT_APPEND
-#define VKB_SHADE_OCTANT_APPEND 0
-#endif
-#ifndef VKB_SHADE_EARLY_APPEND
-#define VKB_SHADE_EARLY_APPEND 1
-#endif
 // The job owning a slot (BATCH) or job 0.
 template <bool BATCH>
 __device__ __forceinline__ uint32_t job_of_slot(const PathParams& p, uint32_t slot) { return BATCH ? __ldg(&p.slot_job[slot]) : 0u; }
@@ -752,7 +716,7 @@ template <bool COUNT, bool BATCH, bool W8 = false>
 __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace(PathParams p, int cur) {
     VKB_STACK_DECL_W(W8)
     const uint32_t n = p.counters[cur];
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&p.counters[3], n);
+    if (blockIdx.x == 0 && threadIdx.x == 0) { atomicAdd(&p.counters[3], n); p.counters[13] = 0u; }
     const uint32_t lane = threadIdx.x & 31u;
     TraceCount tc;
     TraceLane<false, COUNT, W8> L;
@@ -1166,11 +1130,98 @@ __device__ __noinline__ void cache_append(const PathParams& p, float3 world, flo
     }
 }
 
+// Before a bounce's shade pass: the rays that left the scene add what they see and end
+// here; the hits' queue indices are packed, a block's in order, into the bounce's spent
+// origin queue (nothing reads the origins after the trace), counted in counters[13].
+// Bound by the latency of the queue reads (18% issue).  With the misses in the shade kernel
+// a shade warp ran its long hit path for the few of its lanes that hit: 19, 8 and 11 of 32 at
+// bounces 0, 1, 2 of a 256x256 16 spp still, 23 and 6 in a batch of 24 previews, and each
+// warp's instruction stream also missed the instruction cache more.  Packed: 25, 20 and 27,
+// 20 lanes; shade 354 -> 27 + 233 us and 238 -> 18 + 102 us on that still's bounces 0 and 1,
+// 8.06 -> 0.73 + 3.25 ms and 3.48 -> 0.22 + 0.37 ms on the batch's.
+// The bounce's queue counters are reset here too: no kernel reads them between their last
+// reader and this one.
+constexpr int SPLIT_BLOCK = 512;
+template <bool BATCH, bool EXT>
+__global__ void __launch_bounds__(SPLIT_BLOCK) k_split(const __grid_constant__ PathParams p, int cur) {
+    __shared__ uint32_t warp_hits[SPLIT_BLOCK / 32], base;
+    if (blockIdx.x == 0 && threadIdx.x == 0) { p.counters[cur ^ 1] = 0u; p.counters[2] = 0u; p.counters[11] = 0u; p.counters[12] = 0u; }
+    const uint32_t n = p.counters[cur], lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t* hits = reinterpret_cast<uint32_t*>(p.ray_o[cur]);
+    for (uint32_t first = blockIdx.x * SPLIT_BLOCK; first < n; first += gridDim.x * SPLIT_BLOCK) {
+        const uint32_t i = first + threadIdx.x;
+        const uint32_t inst = i < n ? p.hit_inst[i] : 0xffffffffu;
+        const bool hit = inst != 0xffffffffu;
+        const uint32_t mask = __ballot_sync(0xffffffffu, hit);
+        if (lane == 0u) warp_hits[warp] = uint32_t(__popc(mask));
+        __syncthreads();
+        if (warp == 0u) {
+            const uint32_t own = lane < SPLIT_BLOCK / 32 ? warp_hits[lane] : 0u;
+            uint32_t sum = own;
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, sum, off);
+                if (lane >= uint32_t(off)) sum += v;
+            }
+            if (lane < SPLIT_BLOCK / 32) warp_hits[lane] = sum - own;
+            if (lane == 31u) base = sum ? atomicAdd(&p.counters[13], sum) : 0u;
+        }
+        __syncthreads();
+        if (hit) hits[base + warp_hits[warp] + uint32_t(__popc(mask & ((1u << lane) - 1u)))] = i;
+        __syncthreads();   // the next pass writes warp_hits and base
+        if (i >= n) continue;
+        const bool ids = !BATCH ? p.job0.primary_ids != nullptr : true;
+        if (hit && !ids) continue;
+        const float4 rd = p.ray_d[cur][i];
+        const uint32_t slot = __float_as_uint(rd.w);
+        const Job& J = BATCH ? p.jobs[job_of_slot<true>(p, slot)] : p.job0;
+        const float4 T = p.thr[slot];
+        const uint32_t meta = __float_as_uint(T.w), bounce = meta & 0xffu;
+        if (J.primary_ids && bounce == 0u) {
+            const uint32_t local = slot - J.slot_base, pixel = local % J.npix;
+            if (J.wave_first + local / J.npix == J.first_sample) {
+                J.primary_ids[2 * pixel] = inst;
+                J.primary_ids[2 * pixel + 1] = hit ? __float_as_uint(__ldg(&J.sv.blas_tris[3u * size_t(__float_as_uint(p.hit[i].w))]).w) : 0xffffffffu;
+            }
+        }
+        if (hit) continue;
+        // Miss: path.slang:1484-1512 with the constant world light and camera-visible suns.
+        const uint32_t ray_event = bounce == 0 ? VKB_RAY_CAMERA : ((meta >> 24) & 0x3fu);
+        const float limit = bounce == 0 ? J.clamp_direct : J.clamp_indirect;
+        const float4 R = p.rad[slot];
+        const float3 dir = f3(rd.x, rd.y, rd.z), thr = f3(T.x, T.y, T.z);
+        float3 rad = f3(R.x, R.y, R.z);
+        uint32_t dropped = __float_as_uint(R.w);
+        float3 sky;
+        if (ray_event == VKB_RAY_CAMERA && !J.env.camera_sees_environment) sky = get3(J.env.background);
+        else {
+            sky = EXT ? env_radiance(J, dir) : get3(J.env.radiance);
+            if (ray_event == VKB_RAY_CAMERA)
+                for (uint32_t l = 0; l < J.num_lights; ++l) {
+                    const vkb_light& L = J.lights[l];
+                    if (L.position[3] != 0.f || !(L.shadow_offsets[0] & VKB_RAY_CAMERA)) continue;
+                    sky = sky + emitter_eval(L, f3(0.f), dir).radiance;
+                }
+        }
+        if (EXT && J.env_w && bounce > 0u) {
+            // path.slang:1463: an escape after a BSDF sample, weighed against the
+            // environment strategy.
+            const float prev = p.prev[slot].w;
+            if (prev > 0.f) sky = sky * mis_power(prev, env_density(J, dir));
+        }
+        rad = rad + clamp_sample(thr * sky, limit, dropped);
+        p.rad[slot] = make_float4(rad.x, rad.y, rad.z, __uint_as_float(dropped));
+    }
+}
+
 // integrate's per-vertex body (path.slang:1340-1709) for one queued extension hit.
 // The parameter block is __grid_constant__: `J = p.job0` then refers to it in place
 // (a plain by-value parameter that is referenced gets copied to a 736-byte local frame
 // per thread); one block of 512 per SM (128 registers, a small spill) measured faster
-// than 3 blocks of 128 at 158 registers, 4 blocks of 128 and 2 blocks of 256.
+// than 3 blocks of 128 at 158 registers, 4 blocks of 128 and 2 blocks of 256 (their warps
+// start together and share the instruction cache: 5.77 / 5.90 / 6.14 ms at 512 / 256 / 128
+// for a 641x359 still).  Entries are appended where they are made (the threads of a warp
+// that get there together share one atomic), so no queue entry stays live to the end of the
+// loop body.
 #ifndef VKB_SHADE_BLOCK
 #define VKB_SHADE_BLOCK 512
 #endif
@@ -1183,296 +1234,241 @@ constexpr int SHADE_BLOCK = VKB_SHADE_BLOCK;
 template <bool BATCH, bool EXT>
 __global__ void __launch_bounds__(VKB_SHADE_BLOCK, VKB_SHADE_MIN_BLOCKS) k_shade(const __grid_constant__ PathParams p, int cur) {
     const int nxt = cur ^ 1;
-    uint32_t n = p.counters[cur];
-    uint32_t loop_end = (n + blockDim.x - 1) / blockDim.x * blockDim.x;  // whole warps stay in the loop for ballots
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < loop_end; i += gridDim.x * blockDim.x) {
-        bool active = i < n;
-        bool push_ray = false, push_shadow = false;
-        float4 new_o, new_d, sh_o, sh_d, sh_c;
-        uint32_t slot = 0;
-        if (active) {
-            float4 ro = p.ray_o[cur][i], rd = p.ray_d[cur][i];
-            slot = __float_as_uint(rd.w);
-            const Job& J = BATCH ? p.jobs[job_of_slot<true>(p, slot)] : p.job0;
-            float3 dir = f3(rd.x, rd.y, rd.z);
-            float4 hh = p.hit[i];
-            uint32_t inst = p.hit_inst[i];
-            float4 T = p.thr[slot], R = p.rad[slot];
-            uint2 rg = p.rng[slot];
-            uint32_t meta = __float_as_uint(T.w);
-            uint32_t bounce = meta & 0xffu, diffuse = (meta >> 8) & 0xffu, glossy = (meta >> 16) & 0xffu;
-            uint32_t ray_event = bounce == 0 ? VKB_RAY_CAMERA : ((meta >> 24) & 0x3fu);
-            float3 thr = f3(T.x, T.y, T.z), rad = f3(R.x, R.y, R.z);
-            uint32_t dropped = __float_as_uint(R.w), rng = rg.x, pseed = rg.y;
-            uint32_t local = slot - J.slot_base;
-            uint32_t pixel = local % J.npix, sidx = J.wave_first + local / J.npix;
-            float limit = bounce == 0 ? J.clamp_direct : J.clamp_indirect;
-            if (J.primary_ids && bounce == 0 && sidx == J.first_sample) {
-                J.primary_ids[2 * pixel] = hh.x >= 0.f ? inst : 0xffffffffu;
-                J.primary_ids[2 * pixel + 1] = hh.x >= 0.f ? __float_as_uint(__ldg(&J.sv.blas_tris[3u * size_t(__float_as_uint(hh.w))]).w) : 0xffffffffu;
+    const uint32_t n = p.counters[13];
+    const uint32_t* hits = reinterpret_cast<const uint32_t*>(p.ray_o[cur]);
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const uint32_t i = hits[k];
+        const float4 rd = p.ray_d[cur][i];
+        const uint32_t slot = __float_as_uint(rd.w);
+        const Job& J = BATCH ? p.jobs[job_of_slot<true>(p, slot)] : p.job0;
+        const float3 dir = f3(rd.x, rd.y, rd.z);
+        const float4 hh = p.hit[i];
+        const uint32_t inst = p.hit_inst[i];
+        float4 T = p.thr[slot], R = p.rad[slot];
+        uint2 rg = p.rng[slot];
+        uint32_t meta = __float_as_uint(T.w);
+        uint32_t bounce = meta & 0xffu, diffuse = (meta >> 8) & 0xffu, glossy = (meta >> 16) & 0xffu;
+        float3 thr = f3(T.x, T.y, T.z), rad = f3(R.x, R.y, R.z);
+        uint32_t dropped = __float_as_uint(R.w), rng = rg.x, pseed = rg.y;
+        uint32_t local = slot - J.slot_base;
+        uint32_t sidx = J.wave_first + local / J.npix;
+        float limit = bounce == 0 ? J.clamp_direct : J.clamp_indirect;
+        uint32_t vtx = bounce;
+        float4 sc = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 0));   // path_scatter
+        Surface s = hit_surface(J, inst, __float_as_uint(hh.w), hh.y, hh.z, dir);
+        const vkb_material& mt = J.materials[__ldg(&J.inst_info[inst]).y];
+        Closure c;
+        c.base_color = get3(mt.base_color); c.base_weight = mt.base_weight; c.base_metalness = mt.base_metalness;
+        c.specular_color = get3(mt.specular_color); c.specular_weight = mt.specular_weight;
+        c.specular_roughness = mt.specular_roughness; c.specular_ior = mt.specular_ior; c.optical_ior = 0.f;
+        c.n = s.geometric;
+        boundary_closure_air(c);
+        float3 view = -dir;
+        if (EXT && mt.emission_luminance > 0.f && ((mt.flags & 2u) || s.entering)) {
+            // Surface emission (path.slang:1580-1591) on the side the material covers,
+            // weighed against the mesh strategy after a BSDF sample.
+            const float3 emitted = get3(mt.emission_color) * mt.emission_luminance;
+            float mis = 1.f;
+            if (bounce > 0u && J.em_tris) {
+                const float4 pv = p.prev[slot];
+                if (pv.w > 0.f) {
+                    const uint32_t tri = __float_as_uint(hh.w);
+                    const float4* tp = J.sv.blas_tris + 3u * size_t(tri);
+                    const float4 q0 = __ldg(tp), q1 = __ldg(tp + 1), q2 = __ldg(tp + 2);
+                    const float4 M[3] = {__ldg(&J.o2w[3 * inst]), __ldg(&J.o2w[3 * inst + 1]), __ldg(&J.o2w[3 * inst + 2])};
+                    const float3 e1 = mvec(M, f3(q1.x - q0.x, q1.y - q0.y, q1.z - q0.z)), e2 = mvec(M, f3(q2.x - q0.x, q2.y - q0.y, q2.z - q0.z));
+                    const float area = length(cross(e1, e2)) * 0.5f;
+                    mis = mis_power(pv.w, mesh_pdf(J, inst, __float_as_uint(q0.w), area, f3(pv.x, pv.y, pv.z), s.world, s.face));
+                }
             }
-            if (!(hh.x >= 0.f)) {
-                // Miss: path.slang:1484-1512 with the constant world light and camera-visible suns.
-                float3 sky;
-                if (ray_event == VKB_RAY_CAMERA && !J.env.camera_sees_environment) sky = get3(J.env.background);
-                else {
-                    sky = EXT ? env_radiance(J, dir) : get3(J.env.radiance);
-                    if (ray_event == VKB_RAY_CAMERA)
-                        for (uint32_t l = 0; l < J.num_lights; ++l) {
-                            const vkb_light& L = J.lights[l];
-                            if (L.position[3] != 0.f || !(L.shadow_offsets[0] & VKB_RAY_CAMERA)) continue;
-                            sky = sky + emitter_eval(L, f3(0.f), dir).radiance;
-                        }
-                }
-                if (EXT && J.env_w && bounce > 0u) {
-                    // path.slang:1463: an escape after a BSDF sample, weighed against the
-                    // environment strategy.
-                    const float prev = p.prev[slot].w;
-                    if (prev > 0.f) sky = sky * mis_power(prev, env_density(J, dir));
-                }
-                rad = rad + clamp_sample(thr * sky, limit, dropped);
-            } else {
-                uint32_t vtx = bounce;
-                float4 sc = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 0));   // path_scatter
-                Surface s = hit_surface(J, inst, __float_as_uint(hh.w), hh.y, hh.z, dir);
-                const vkb_material& mt = J.materials[__ldg(&J.inst_info[inst]).y];
-                Closure c;
-                c.base_color = get3(mt.base_color); c.base_weight = mt.base_weight; c.base_metalness = mt.base_metalness;
-                c.specular_color = get3(mt.specular_color); c.specular_weight = mt.specular_weight;
-                c.specular_roughness = mt.specular_roughness; c.specular_ior = mt.specular_ior; c.optical_ior = 0.f;
-                c.n = s.geometric;
-                boundary_closure_air(c);
-                float3 view = -dir;
-                if (EXT && mt.emission_luminance > 0.f && ((mt.flags & 2u) || s.entering)) {
-                    // Surface emission (path.slang:1580-1591) on the side the material covers,
-                    // weighed against the mesh strategy after a BSDF sample.
-                    const float3 emitted = get3(mt.emission_color) * mt.emission_luminance;
-                    float mis = 1.f;
-                    if (bounce > 0u && J.em_tris) {
-                        const float4 pv = p.prev[slot];
-                        if (pv.w > 0.f) {
-                            const uint32_t tri = __float_as_uint(hh.w);
-                            const float4* tp = J.sv.blas_tris + 3u * size_t(tri);
-                            const float4 q0 = __ldg(tp), q1 = __ldg(tp + 1), q2 = __ldg(tp + 2);
-                            const float4 M[3] = {__ldg(&J.o2w[3 * inst]), __ldg(&J.o2w[3 * inst + 1]), __ldg(&J.o2w[3 * inst + 2])};
-                            const float3 e1 = mvec(M, f3(q1.x - q0.x, q1.y - q0.y, q1.z - q0.z)), e2 = mvec(M, f3(q2.x - q0.x, q2.y - q0.y, q2.z - q0.z));
-                            const float area = length(cross(e1, e2)) * 0.5f;
-                            mis = mis_power(pv.w, mesh_pdf(J, inst, __float_as_uint(q0.w), area, f3(pv.x, pv.y, pv.z), s.world, s.face));
+            rad = rad + clamp_sample(thr * emitted * mis, limit, dropped);
+        }
+        // Radiance cache: record this vertex, and at the query vertex stop the path
+        // here (the query kernel adds thr x the cached outgoing radiance).
+        const bool cache_query = p.cache.mode == 1u && bounce >= p.cache.vertex;
+        if (cache_query || (p.cache.mode == 2u && bounce >= 1u)) cache_append(p, s.world, view, s.geometric, c.specular_roughness, c.base_metalness, c.base_color, slot, bounce, thr, rad);
+        if (!cache_query) {
+        float3 iface = dot(s.geometric, view) > 0.f ? s.geometric : s.face;
+        Prepared pr = transport_prepare(p.lut, c, view, s.geometric, iface);
+        BsdfSample smp = transport_sample(c, view, sc.x, sc.y, sc.z, pr);
+        if (!finite3(smp.dir) || !finite3(smp.weight) || !isfinite(smp.pdf)) {
+            meta |= META_NONFINITE;
+        } else {
+            // The image-environment and mesh strategies first: their shadow rays go
+            // to the slot's own buffers at once, so nothing of theirs stays live
+            // across the analytic estimate (the sample groups and the order of the
+            // sums in the shadow kernel do not depend on this order).
+            // environment_next_event (path.slang:1096-1120): a proposal direction,
+            // the diffuse and specular responses MIS-weighted against continuing
+            // there (continuation_mask, path.slang:1003-1010), one visibility ray
+            // to infinity; clamped on its own.
+            bool trace_c = false, trace_d = false;
+            uint32_t cont = 0u;
+            if (EXT && bounce < J.bounces[0]) {
+                if (diffuse < J.bounces[1]) cont |= VKB_RAY_DIFFUSE;
+                if (glossy < J.bounces[2] && (diffuse == 0u || (J.caustics & 1u))) cont |= VKB_RAY_SPECULAR;
+            }
+            if (EXT && J.env_w) {
+                const float4 eu = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 3));   // path_environment
+                float epdf = 0.f;
+                const float3 edir = env_sample(J, eu.x, eu.y, epdf);
+                float3 ev = f3(0.f);
+                if (epdf > 0.f) {
+                    const float3 emitted = env_radiance(J, edir);
+                    if (maxc(emitted) > 0.f) {
+                        #pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            const uint32_t event = k == 0 ? VKB_RAY_DIFFUSE : VKB_RAY_SPECULAR;
+                            if (!event_hemisphere(event, edir, s.face, s.geometric)) continue;
+                            const float3 response = eval_mask(c, view, edir, event, pr);
+                            if (maxc(response) <= 0.f) continue;
+                            const float bpdf = (cont & event) ? pdf_mask(c, view, edir, event, pr) : 0.f;
+                            ev = ev + emitted * response * (mis_power(epdf, bpdf) / epdf);
                         }
                     }
-                    rad = rad + clamp_sample(thr * emitted * mis, limit, dropped);
                 }
-                // Radiance cache: record this vertex, and at the query vertex stop the path
-                // here (the query kernel adds thr x the cached outgoing radiance).
-                const bool cache_query = p.cache.mode == 1u && bounce >= p.cache.vertex;
-                if (cache_query || (p.cache.mode == 2u && bounce >= 1u)) cache_append(p, s.world, view, s.geometric, c.specular_roughness, c.base_metalness, c.base_color, slot, bounce, thr, rad);
-                if (!cache_query) {
-                float3 iface = dot(s.geometric, view) > 0.f ? s.geometric : s.face;
-                Prepared pr = transport_prepare(p.lut, c, view, s.geometric, iface);
-                BsdfSample smp = transport_sample(c, view, sc.x, sc.y, sc.z, pr);
-                if (!finite3(smp.dir) || !finite3(smp.weight) || !isfinite(smp.pdf)) {
-                    meta |= META_NONFINITE;
-                } else {
-                    // The image-environment and mesh strategies first: their shadow rays go
-                    // to the slot's own buffers at once, so nothing of theirs stays live
-                    // across the analytic estimate (the sample groups and the order of the
-                    // sums in the shadow kernel do not depend on this order).
-                    // environment_next_event (path.slang:1096-1120): a proposal direction,
-                    // the diffuse and specular responses MIS-weighted against continuing
-                    // there (continuation_mask, path.slang:1003-1010), one visibility ray
-                    // to infinity; clamped on its own.
-                    bool trace_c = false, trace_d = false;
-                    uint32_t cont = 0u;
-                    if (EXT && bounce < J.bounces[0]) {
-                        if (diffuse < J.bounces[1]) cont |= VKB_RAY_DIFFUSE;
-                        if (glossy < J.bounces[2] && (diffuse == 0u || (J.caustics & 1u))) cont |= VKB_RAY_SPECULAR;
-                    }
-                    if (EXT && J.env_w) {
-                        const float4 eu = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 3));   // path_environment
-                        float epdf = 0.f;
-                        const float3 edir = env_sample(J, eu.x, eu.y, epdf);
-                        float3 ev = f3(0.f);
-                        if (epdf > 0.f) {
-                            const float3 emitted = env_radiance(J, edir);
-                            if (maxc(emitted) > 0.f) {
+                if (any_nonzero(ev)) {
+                    const float3 oc = path_origin(s, edir), cc = thr * ev;
+                    p.sc_o[slot] = make_float4(oc.x, oc.y, oc.z, FP32_MAX);
+                    p.sc_d[slot] = make_float4(edir.x, edir.y, edir.z, 0.f);
+                    p.sc_c[slot] = make_float4(cc.x, cc.y, cc.z, 0.f);
+                    trace_c = true;
+                }
+            }
+            if (EXT && J.em_tris) {
+                // mesh_next_event (path.slang:1121-1167), constant emission: a point on a
+                // source triangle, the diffuse and specular responses MIS-weighted against
+                // continuing there, one visibility ray between the offset end points.
+                const float4 g = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 2));   // path_triangle
+                uint32_t ei, ep; float b1, b2;
+                if (em_sample(J, g.z, g.x, g.y, ei, ep, b1, b2)) {
+                    const EmGeometry eg = em_geometry(J, ei, ep, b1, b2);
+                    const float3 delta = eg.point - s.world;
+                    const float distance = length(delta);
+                    if (distance > 0.f) {
+                        const float3 axis = delta / distance;
+                        const float mpdf = mesh_pdf(J, ei, ep, eg.area, s.world, eg.point, eg.face);
+                        const vkb_material& em = J.materials[__ldg(&J.inst_info[ei]).y];
+                        const bool front = dot(eg.face, axis) < 0.f;
+                        const float3 emitted = get3(em.emission_color) * em.emission_luminance;
+                        if (mpdf > 0.f && ((em.flags & 2u) || front) && maxc(emitted) > 0.f) {
+                            const float3 start = path_origin(s, axis);
+                            const float3 end = surface_ray_origin(eg.point, eg.error, front ? eg.face : -eg.face, -axis);
+                            const float3 connection = end - start;
+                            const float extent = length(connection);
+                            float3 response = f3(0.f);
+                            if (extent > 0.f) {
                                 #pragma unroll
                                 for (int k = 0; k < 2; ++k) {
                                     const uint32_t event = k == 0 ? VKB_RAY_DIFFUSE : VKB_RAY_SPECULAR;
-                                    if (!event_hemisphere(event, edir, s.face, s.geometric)) continue;
-                                    const float3 response = eval_mask(c, view, edir, event, pr);
-                                    if (maxc(response) <= 0.f) continue;
-                                    const float bpdf = (cont & event) ? pdf_mask(c, view, edir, event, pr) : 0.f;
-                                    ev = ev + emitted * response * (mis_power(epdf, bpdf) / epdf);
+                                    if (!event_hemisphere(event, axis, s.face, s.geometric)) continue;
+                                    const float3 f = eval_mask(c, view, axis, event, pr);
+                                    if (maxc(f) <= 0.f) continue;
+                                    const float bpdf = (cont & event) ? pdf_mask(c, view, axis, event, pr) : 0.f;
+                                    response = response + f * mis_power(mpdf, bpdf);
                                 }
                             }
-                        }
-                        if (any_nonzero(ev)) {
-                            const float3 oc = path_origin(s, edir), cc = thr * ev;
-                            p.sc_o[slot] = make_float4(oc.x, oc.y, oc.z, FP32_MAX);
-                            p.sc_d[slot] = make_float4(edir.x, edir.y, edir.z, 0.f);
-                            p.sc_c[slot] = make_float4(cc.x, cc.y, cc.z, 0.f);
-                            trace_c = true;
-                        }
-                    }
-                    if (EXT && J.em_tris) {
-                        // mesh_next_event (path.slang:1121-1167), constant emission: a point on a
-                        // source triangle, the diffuse and specular responses MIS-weighted against
-                        // continuing there, one visibility ray between the offset end points.
-                        const float4 g = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 2));   // path_triangle
-                        uint32_t ei, ep; float b1, b2;
-                        if (em_sample(J, g.z, g.x, g.y, ei, ep, b1, b2)) {
-                            const EmGeometry eg = em_geometry(J, ei, ep, b1, b2);
-                            const float3 delta = eg.point - s.world;
-                            const float distance = length(delta);
-                            if (distance > 0.f) {
-                                const float3 axis = delta / distance;
-                                const float mpdf = mesh_pdf(J, ei, ep, eg.area, s.world, eg.point, eg.face);
-                                const vkb_material& em = J.materials[__ldg(&J.inst_info[ei]).y];
-                                const bool front = dot(eg.face, axis) < 0.f;
-                                const float3 emitted = get3(em.emission_color) * em.emission_luminance;
-                                if (mpdf > 0.f && ((em.flags & 2u) || front) && maxc(emitted) > 0.f) {
-                                    const float3 start = path_origin(s, axis);
-                                    const float3 end = surface_ray_origin(eg.point, eg.error, front ? eg.face : -eg.face, -axis);
-                                    const float3 connection = end - start;
-                                    const float extent = length(connection);
-                                    float3 response = f3(0.f);
-                                    if (extent > 0.f) {
-                                        #pragma unroll
-                                        for (int k = 0; k < 2; ++k) {
-                                            const uint32_t event = k == 0 ? VKB_RAY_DIFFUSE : VKB_RAY_SPECULAR;
-                                            if (!event_hemisphere(event, axis, s.face, s.geometric)) continue;
-                                            const float3 f = eval_mask(c, view, axis, event, pr);
-                                            if (maxc(f) <= 0.f) continue;
-                                            const float bpdf = (cont & event) ? pdf_mask(c, view, axis, event, pr) : 0.f;
-                                            response = response + f * mis_power(mpdf, bpdf);
-                                        }
-                                    }
-                                    if (any_nonzero(response)) {
-                                        const float3 md = thr * (response * emitted / mpdf), cdir = connection / extent;
-                                        p.sd_o[slot] = make_float4(start.x, start.y, start.z, extent);
-                                        p.sd_d[slot] = make_float4(cdir.x, cdir.y, cdir.z, 0.f);
-                                        p.sd_c[slot] = make_float4(md.x, md.y, md.z, 0.f);
-                                        trace_d = true;
-                                    }
-                                }
+                            if (any_nonzero(response)) {
+                                const float3 md = thr * (response * emitted / mpdf), cdir = connection / extent;
+                                p.sd_o[slot] = make_float4(start.x, start.y, start.z, extent);
+                                p.sd_d[slot] = make_float4(cdir.x, cdir.y, cdir.z, 0.f);
+                                p.sd_c[slot] = make_float4(md.x, md.y, md.z, 0.f);
+                                trace_d = true;
                             }
                         }
-                    }
-                    // next_event (path.slang:851-951): one analytic light, two estimators.
-                    float3 va = f3(0.f), vb = f3(0.f);
-                    bool trace_a = false, has_b = false, trace_b = false;
-                    float3 oa, da, ob, db; float la = 0.f, lb = 0.f;
-                    if (J.num_lights > 0) {
-                        float4 u = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 1));   // path_light
-                        float probability;
-                        uint32_t li = tree_pick(J.tree, J.tree_nodes, s.world, u.z, u.w, probability);
-                        if (probability > 0.f && li < J.num_lights) {
-                            const vkb_light& L = J.lights[li];
-                            uint32_t contribution = L.shadow_offsets[VKB_LIGHT_CONTRIBUTION_WORD];
-                            bool shadowed = (L.shadow_offsets[VKB_LIGHT_RAY_WORD] & VKB_LIGHT_RAY_SHADOWED) != 0u;
-                            if ((contribution & VKB_LIGHT_LINK_ALL) || L.shadow_offsets[VKB_LIGHT_LINK_WORD]) {
-                                LightSample src = emitter_sample(L, s.world, u.x, u.y);
-                                float3 power = src.delta ? src.radiance : (src.pdf > 0.f ? src.radiance / src.pdf : f3(0.f));
-                                va = analytic_mis_response(c, view, src.dir, s.face, contribution, src.pdf, pr) * power / probability;
-                                va = light_threshold(va, J.light_threshold, rng);
-                                if (any_nonzero(va) && shadowed) {
-                                    oa = path_origin(s, src.dir);
-                                    ray_connection(oa, s.world, src.dir, src.distance, da, la);
-                                    trace_a = true;
-                                }
-                                bool continuation = (contribution & smp.event) && event_hemisphere(smp.event, smp.dir, s.face, s.geometric);
-                                if (continuation && dot(smp.dir, smp.dir) > 0.f) {
-                                    EmitterEval e = emitter_eval(L, s.world, smp.dir);
-                                    if (e.pdf > 0.f) {
-                                        float w = smp.pdf > 0.f ? mis_power(smp.pdf, e.pdf) : 1.f;
-                                        vb = light_threshold(smp.weight * e.radiance * (w / probability), J.light_threshold, rng);
-                                        if (any_nonzero(vb)) {
-                                            has_b = true;
-                                            if (shadowed) {
-                                                ob = path_origin(s, smp.dir);
-                                                ray_connection(ob, s.world, smp.dir, e.distance, db, lb);
-                                                trace_b = true;
-                                            }
-                                        }
-                                    }
-                                }
-                            }
-                        }
-                    }
-                    float3 ca = thr * va, cb = thr * vb;
-                    if (trace_a || trace_b || trace_c || trace_d) {
-                        push_shadow = true;
-                        uint32_t flags = (trace_a ? SH_TRACE_A : 0u) | (has_b ? SH_HAS_B : 0u) | (trace_b ? SH_TRACE_B : 0u) | (bounce == 0 ? SH_DIRECT : 0u) |
-                                         (trace_c ? SH_HAS_C : 0u) | (trace_d ? SH_HAS_D : 0u);
-                        sh_o = make_float4(oa.x, oa.y, oa.z, la);
-                        sh_d = make_float4(da.x, da.y, da.z, __uint_as_float(slot));
-                        sh_c = make_float4(ca.x, ca.y, ca.z, __uint_as_float(flags));
-                        if (!trace_a) sh_o = make_float4(0.f, 0.f, 0.f, 0.f);
-#if VKB_SHADE_EARLY_APPEND
-                        {
-                            const uint32_t si = group_append(&p.counters[2]);
-                            p.sa_o[si] = sh_o; p.sa_d[si] = sh_d; p.sa_c[si] = sh_c;
-                            push_shadow = false;
-                        }
-#endif
-                        if (has_b) {
-                            p.sb_c[slot] = make_float4(cb.x, cb.y, cb.z, 0.f);
-                            if (trace_b) { p.sb_o[slot] = make_float4(ob.x, ob.y, ob.z, lb); p.sb_d[slot] = make_float4(db.x, db.y, db.z, 0.f); }
-                        }
-                    } else {
-                        rad = rad + clamp_sample(ca + cb, limit, dropped);
-                    }
-                    // Continuation (path.slang:1683-1708).
-                    bool go = bounce < J.bounces[0];
-                    uint32_t event = smp.event;
-                    if (go) {
-                        if (event == VKB_RAY_DIFFUSE) { if (diffuse++ >= J.bounces[1]) go = false; }
-                        else if (event == VKB_RAY_SPECULAR) { if (glossy++ >= J.bounces[2] || (diffuse > 0 && !(J.caustics & 1u))) go = false; }
-                        else go = false;
-                    }
-                    if (go && !event_hemisphere(event, smp.dir, s.face, s.geometric)) go = false;
-                    if (go) {
-                        thr = thr * smp.weight;
-                        if (!finite3(thr)) { meta |= META_NONFINITE; go = false; }
-                        else if (maxc(thr) <= 0.f) go = false;
-                    }
-                    if (go && bounce >= ROULETTE_START) {
-                        float survive = clampf(maxc(thr), ROULETTE_MIN, ROULETTE_MAX);
-                        float4 dec = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 4));
-                        if (dec.z > survive) go = false;
-                        else thr = thr / survive;
-                    }
-                    if (go) {
-                        float3 o = path_origin(s, smp.dir);
-                        new_o = make_float4(o.x, o.y, o.z, FP32_MAX);
-                        new_d = make_float4(smp.dir.x, smp.dir.y, smp.dir.z, __uint_as_float(slot));
-                        push_ray = true;
-                        if (EXT) p.prev[slot] = make_float4(s.world.x, s.world.y, s.world.z, smp.pdf);
-#if VKB_SHADE_EARLY_APPEND
-                        {
-#if VKB_SHADE_OCTANT_APPEND
-                            const uint32_t oct = (smp.dir.x < 0.f ? 1u : 0u) | (smp.dir.y < 0.f ? 2u : 0u) | (smp.dir.z < 0.f ? 4u : 0u);
-                            const uint32_t ri = group_append_by_key(&p.counters[nxt], oct);
-#else
-                            const uint32_t ri = group_append(&p.counters[nxt]);
-#endif
-                            p.ray_o[nxt][ri] = new_o; p.ray_d[nxt][ri] = new_d;
-                            push_ray = false;
-                        }
-#endif
-                        meta = (meta & META_NONFINITE) | ((bounce + 1u) & 0xffu) | ((diffuse & 0xffu) << 8) | ((glossy & 0xffu) << 16) | ((event & 0x3fu) << 24);
                     }
                 }
-                }  // !cache_query
             }
-            p.thr[slot] = make_float4(thr.x, thr.y, thr.z, __uint_as_float(meta));
-            p.rad[slot] = make_float4(rad.x, rad.y, rad.z, __uint_as_float(dropped));
-            p.rng[slot] = make_uint2(rng, pseed);
+            // next_event (path.slang:851-951): one analytic light, two estimators.
+            float3 va = f3(0.f), vb = f3(0.f);
+            bool trace_a = false, has_b = false, trace_b = false;
+            float3 oa, da, ob, db; float la = 0.f, lb = 0.f;
+            if (J.num_lights > 0) {
+                float4 u = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 1));   // path_light
+                float probability;
+                uint32_t li = tree_pick(J.tree, J.tree_nodes, s.world, u.z, u.w, probability);
+                if (probability > 0.f && li < J.num_lights) {
+                    const vkb_light& L = J.lights[li];
+                    uint32_t contribution = L.shadow_offsets[VKB_LIGHT_CONTRIBUTION_WORD];
+                    bool shadowed = (L.shadow_offsets[VKB_LIGHT_RAY_WORD] & VKB_LIGHT_RAY_SHADOWED) != 0u;
+                    if ((contribution & VKB_LIGHT_LINK_ALL) || L.shadow_offsets[VKB_LIGHT_LINK_WORD]) {
+                        LightSample src = emitter_sample(L, s.world, u.x, u.y);
+                        float3 power = src.delta ? src.radiance : (src.pdf > 0.f ? src.radiance / src.pdf : f3(0.f));
+                        va = analytic_mis_response(c, view, src.dir, s.face, contribution, src.pdf, pr) * power / probability;
+                        va = light_threshold(va, J.light_threshold, rng);
+                        if (any_nonzero(va) && shadowed) {
+                            oa = path_origin(s, src.dir);
+                            ray_connection(oa, s.world, src.dir, src.distance, da, la);
+                            trace_a = true;
+                        }
+                        bool continuation = (contribution & smp.event) && event_hemisphere(smp.event, smp.dir, s.face, s.geometric);
+                        if (continuation && dot(smp.dir, smp.dir) > 0.f) {
+                            EmitterEval e = emitter_eval(L, s.world, smp.dir);
+                            if (e.pdf > 0.f) {
+                                float w = smp.pdf > 0.f ? mis_power(smp.pdf, e.pdf) : 1.f;
+                                vb = light_threshold(smp.weight * e.radiance * (w / probability), J.light_threshold, rng);
+                                if (any_nonzero(vb)) {
+                                    has_b = true;
+                                    if (shadowed) {
+                                        ob = path_origin(s, smp.dir);
+                                        ray_connection(ob, s.world, smp.dir, e.distance, db, lb);
+                                        trace_b = true;
+                                    }
+                                }
+                            }
+                        }
+                    }
+                }
+            }
+            float3 ca = thr * va, cb = thr * vb;
+            if (trace_a || trace_b || trace_c || trace_d) {
+                uint32_t flags = (trace_a ? SH_TRACE_A : 0u) | (has_b ? SH_HAS_B : 0u) | (trace_b ? SH_TRACE_B : 0u) | (bounce == 0 ? SH_DIRECT : 0u) |
+                                 (trace_c ? SH_HAS_C : 0u) | (trace_d ? SH_HAS_D : 0u);
+                const uint32_t si = group_append(&p.counters[2]);
+                p.sa_o[si] = trace_a ? make_float4(oa.x, oa.y, oa.z, la) : make_float4(0.f, 0.f, 0.f, 0.f);
+                p.sa_d[si] = make_float4(da.x, da.y, da.z, __uint_as_float(slot));
+                p.sa_c[si] = make_float4(ca.x, ca.y, ca.z, __uint_as_float(flags));
+                if (has_b) {
+                    p.sb_c[slot] = make_float4(cb.x, cb.y, cb.z, 0.f);
+                    if (trace_b) { p.sb_o[slot] = make_float4(ob.x, ob.y, ob.z, lb); p.sb_d[slot] = make_float4(db.x, db.y, db.z, 0.f); }
+                }
+            } else {
+                rad = rad + clamp_sample(ca + cb, limit, dropped);
+            }
+            // Continuation (path.slang:1683-1708).
+            bool go = bounce < J.bounces[0];
+            uint32_t event = smp.event;
+            if (go) {
+                if (event == VKB_RAY_DIFFUSE) { if (diffuse++ >= J.bounces[1]) go = false; }
+                else if (event == VKB_RAY_SPECULAR) { if (glossy++ >= J.bounces[2] || (diffuse > 0 && !(J.caustics & 1u))) go = false; }
+                else go = false;
+            }
+            if (go && !event_hemisphere(event, smp.dir, s.face, s.geometric)) go = false;
+            if (go) {
+                thr = thr * smp.weight;
+                if (!finite3(thr)) { meta |= META_NONFINITE; go = false; }
+                else if (maxc(thr) <= 0.f) go = false;
+            }
+            if (go && bounce >= ROULETTE_START) {
+                float survive = clampf(maxc(thr), ROULETTE_MIN, ROULETTE_MAX);
+                float4 dec = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 4));
+                if (dec.z > survive) go = false;
+                else thr = thr / survive;
+            }
+            if (go) {
+                float3 o = path_origin(s, smp.dir);
+                if (EXT) p.prev[slot] = make_float4(s.world.x, s.world.y, s.world.z, smp.pdf);
+                const uint32_t ri = group_append(&p.counters[nxt]);
+                p.ray_o[nxt][ri] = make_float4(o.x, o.y, o.z, FP32_MAX);
+                p.ray_d[nxt][ri] = make_float4(smp.dir.x, smp.dir.y, smp.dir.z, __uint_as_float(slot));
+                meta = (meta & META_NONFINITE) | ((bounce + 1u) & 0xffu) | ((diffuse & 0xffu) << 8) | ((glossy & 0xffu) << 16) | ((event & 0x3fu) << 24);
+            }
         }
-        uint32_t ri = warp_append(&p.counters[nxt], push_ray);
-        if (push_ray) { p.ray_o[nxt][ri] = new_o; p.ray_d[nxt][ri] = new_d; }
-        uint32_t si = warp_append(&p.counters[2], push_shadow);
-        if (push_shadow) { p.sa_o[si] = sh_o; p.sa_d[si] = sh_d; p.sa_c[si] = sh_c; }
+        }  // !cache_query
+    
+        p.thr[slot] = make_float4(thr.x, thr.y, thr.z, __uint_as_float(meta));
+        p.rad[slot] = make_float4(rad.x, rad.y, rad.z, __uint_as_float(dropped));
+        p.rng[slot] = make_uint2(rng, pseed);
     }
 }
 // Seed the first ray queue's count from the wave's path-slot count.
@@ -1524,8 +1520,6 @@ __global__ void k_adaptive_decide(PathParams p) {
     for (int off = 16; off > 0; off >>= 1) skipped += __shfl_xor_sync(0xffffffffu, skipped, off);
     if ((threadIdx.x & 31u) == 0u && skipped) atomicAdd(&p.counters[10], skipped);
 }
-// Zero the next ray queue and the shadow queue before a shade pass.
-__global__ void k_reset_queues(uint32_t* counters, int nxt) { counters[nxt] = 0u; counters[2] = 0u; counters[11] = 0u; counters[12] = 0u; }
 // Denoiser guides of this wave's camera hits (path.slang:1549-1571): per path slot the
 // hit's guide albedo (w = 1: coverage) and shading normal, zero on a miss.  Runs between
 // the bounce-0 closest-hit trace and the shade pass of single-job guide renders.
