@@ -781,14 +781,15 @@ struct CacheLaunch {
 // persistent (a warp takes rays until the counter runs out), so they need the resident
 // blocks and no more: 1920x1080 frames of the flock are equal at 8 and 128 blocks per SM.
 // The shade grid strides; more blocks than are resident balance its load, so it keeps the
-// context's blocks per SM where the wave has that many entries.
+// context's blocks per SM where the wave has that many entries.  Short queues are spread
+// thin (short_share), so a small wave gets a warp for every four of its slots.
 struct WaveGrids {
     int trace, split, shade;
     WaveGrids(const vkb_ctx* c, uint32_t paths) {
         const uint32_t sms = uint32_t(c->sms);
-        trace = int(std::max(1u, std::min((paths + TRACE_BLOCK - 1u) / TRACE_BLOCK, sms * VKB_TRACE_MIN_BLOCKS)));
+        trace = int(std::max(1u, std::min((paths + 15u) / 16u, sms * VKB_TRACE_MIN_BLOCKS)));
         split = int(std::max(1u, std::min((paths + SPLIT_BLOCK - 1u) / SPLIT_BLOCK, sms * 16u)));
-        shade = int(std::max(1u, std::min((paths + SHADE_BLOCK - 1u) / SHADE_BLOCK, sms * uint32_t(c->trace_blocks_per_sm))));
+        shade = int(std::max(std::min((paths + 63u) / 64u, sms), std::min((paths + SHADE_BLOCK - 1u) / SHADE_BLOCK, sms * uint32_t(c->trace_blocks_per_sm))));
     }
 };
 
@@ -839,12 +840,12 @@ void wave_kernels(vkb_ctx* c, const PathParams& p, uint32_t paths, uint32_t boun
         // strategies (two more shadow rays per vertex); the others keep the plain ones.
         if (ext) {
             k_split<BATCH, true><<<grids.split, SPLIT_BLOCK, 0, st>>>(p, cur);
-            k_shade<BATCH, true><<<sgrid, SHADE_BLOCK, 0, st>>>(p, cur);
+            k_shade<BATCH, true><<<sgrid, SHADE_BLOCK, 0, st>>>(p, cur, uint32_t(sms));
             if (w8) launch_shadow<BATCH, true, true>(counted, tgrid, st, p);
             else launch_shadow<BATCH, true, false>(counted, tgrid, st, p);
         } else {
             k_split<BATCH, false><<<grids.split, SPLIT_BLOCK, 0, st>>>(p, cur);
-            k_shade<BATCH, false><<<sgrid, SHADE_BLOCK, 0, st>>>(p, cur);
+            k_shade<BATCH, false><<<sgrid, SHADE_BLOCK, 0, st>>>(p, cur, uint32_t(sms));
             if (w8) launch_shadow<BATCH, false, true>(counted, tgrid, st, p);
             else launch_shadow<BATCH, false, false>(counted, tgrid, st, p);
         }

@@ -699,6 +699,20 @@ __device__ __forceinline__ bool trace_any(const SceneView& sv, RayRef ray, float
 #endif
 static_assert(VKB_TRACE_REFILL >= 1 && VKB_TRACE_REFILL <= 31, "refill threshold in lanes");
 static_assert(VKB_TRACE_NODES >= 0 && VKB_TRACE_NODES <= 31, "node threshold in lanes");
+// Lanes of each warp that take an entry when a queue of n entries is shorter than the lanes
+// of `warps` resident warps (0: it is not).  A short queue takes as long as its longest
+// entry, and an entry's steps wait for every branch its warp's other lanes take: n entries
+// spread over all the warps, down to one each, finish before n / 32 full warps do (128x128
+// 1 spp: 614 us full, 572 / 543 / 508 us at no fewer than 8 / 4 / 1 entries a warp; the late
+// bounces of every render are such queues: the 1080p 64 spp flock frame 386.8 -> 376.8 ms).
+// Entry w * share + lane is warp w's, so there is nothing left to take from the counter.
+__device__ __forceinline__ uint32_t short_share(uint32_t n, uint32_t warps) {
+    const uint32_t share = (n + warps - 1u) / warps;
+    return share <= 32u ? max(share, 1u) : 0u;
+}
+__device__ __forceinline__ uint32_t share_index(uint32_t share) {
+    return (blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u) * share + (threadIdx.x & 31u);
+}
 // Closest hits of the queued rays.  Bound by instruction issue under divergence (issue 56%
 // of cycles, 10 of 32 lanes) behind dependent node fetches.  A ray's steps are ~85% node
 // visits; at two dozen rays a warp nearly always had one lane at a leaf, an instance entry
@@ -723,6 +737,17 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace(Pat
     constexpr uint32_t NONE = 0xffffffffu;
     uint32_t ray = NONE, job = 0;
     bool drained = false;
+    auto take = [&](uint32_t r) {
+        ray = r;
+        if (BATCH) job = job_of_slot<true>(p, __float_as_uint(p.ray_d[cur][r].w));
+        L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.ray_o[cur], p.ray_d[cur], r}, p.ray_o[cur][r].w);
+    };
+    const uint32_t share = short_share(n, gridDim.x * (TRACE_BLOCK / 32u));
+    if (share) {
+        const uint32_t r = share_index(share);
+        if (lane < share && r < n) take(r);
+        drained = true;
+    }
     for (;;) {
         uint32_t act = __ballot_sync(0xffffffffu, !L.done());
         if (act == 0u || (!drained && uint32_t(__popc(act)) <= uint32_t(VKB_TRACE_REFILL))) {
@@ -738,11 +763,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace(Pat
             base = __shfl_sync(0xffffffffu, base, 0);
             drained = base + uint32_t(__popc(idle)) >= n;
             const uint32_t r = base + uint32_t(__popc(idle & ((1u << lane) - 1u)));
-            if (L.done() && r < n) {
-                ray = r;
-                if (BATCH) job = job_of_slot<true>(p, __float_as_uint(p.ray_d[cur][r].w));
-                L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.ray_o[cur], p.ray_d[cur], r}, p.ray_o[cur][r].w);
-            }
+            if (L.done() && r < n) take(r);
         }
         if (L.at_special()) L.special(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.ray_o[cur], p.ray_d[cur], ray}, p.err, &tc, stk);
         do {
@@ -820,7 +841,19 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace_sha
         p.rad[slot] = make_float4(r.x + add.x, r.y + add.y, r.z + add.z, __uint_as_float(dropped));
         e = NONE;
     };
+    auto take = [&](uint32_t r) {
+        e = r;
+        occ = 0u;
+        if (BATCH) job = job_of_slot<true>(p, __float_as_uint(p.sa_d[r].w));
+        if (!begin(0u)) finish();
+    };
     bool drained = false;
+    const uint32_t share = short_share(n, gridDim.x * (TRACE_BLOCK / 32u));
+    if (share) {
+        const uint32_t r = share_index(share);
+        if (lane < share && r < n) take(r);
+        drained = true;
+    }
     for (;;) {
         uint32_t act = __ballot_sync(0xffffffffu, !L.done());
         if (act == 0u || (!drained && uint32_t(__popc(act)) <= uint32_t(VKB_TRACE_REFILL))) {
@@ -838,12 +871,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace_sha
                 base = __shfl_sync(0xffffffffu, base, 0);
                 drained = base + uint32_t(__popc(idle)) >= n;
                 const uint32_t r = base + uint32_t(__popc(idle & ((1u << lane) - 1u)));
-                if (e == NONE && r < n) {
-                    e = r;
-                    occ = 0u;
-                    if (BATCH) job = job_of_slot<true>(p, __float_as_uint(p.sa_d[r].w));
-                    if (!begin(0u)) finish();
-                }
+                if (e == NONE && r < n) take(r);
             }
         }
         if (L.at_special()) {
@@ -1231,12 +1259,18 @@ __global__ void __launch_bounds__(SPLIT_BLOCK) k_split(const __grid_constant__ P
 constexpr int SHADE_BLOCK = VKB_SHADE_BLOCK;
 // EXT: waves with an image environment or emissive meshes (their strategies and the
 // per-slot previous vertex); the plain instantiation carries none of it.
+// resident: the blocks that run at once; a short hit list is spread over their warps.
 template <bool BATCH, bool EXT>
-__global__ void __launch_bounds__(VKB_SHADE_BLOCK, VKB_SHADE_MIN_BLOCKS) k_shade(const __grid_constant__ PathParams p, int cur) {
+__global__ void __launch_bounds__(VKB_SHADE_BLOCK, VKB_SHADE_MIN_BLOCKS) k_shade(const __grid_constant__ PathParams p, int cur, uint32_t resident) {
     const int nxt = cur ^ 1;
     const uint32_t n = p.counters[13];
     const uint32_t* hits = reinterpret_cast<const uint32_t*>(p.ray_o[cur]);
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    if (const uint32_t share = short_share(n, min(gridDim.x, resident) * (SHADE_BLOCK / 32u))) {
+        k = blockIdx.x < resident && (threadIdx.x & 31u) < share ? share_index(share) : n;
+        stride = n;
+    }
+    for (; k < n; k += stride) {
         const uint32_t i = hits[k];
         const float4 rd = p.ray_d[cur][i];
         const uint32_t slot = __float_as_uint(rd.w);
