@@ -449,7 +449,9 @@ struct Job {
     uint32_t spp, seed, bounces[4], caustics, sample_mask;
     float clamp_direct, clamp_indirect, light_threshold;
     uint32_t npix, first_sample;
-    uint32_t wave_first, wave_samples, slot_base, pixel_base;  // this wave
+    // This wave: path slot slot_base + pixel * wave_samples + k is the pixel's sample
+    // wave_first + k, so neighbouring lanes trace one pixel's samples (see k_camera).
+    uint32_t wave_first, wave_samples, slot_base, pixel_base;
     float4* accum; uint32_t* primary_ids; float4* out;
     // Adaptive sampling (path.slang:1792-1837,1963-1966): per-pixel moments (mean, M2 of
     // the accumulated RGBA values) and a state word (bit 0/1: settled at an even/odd
@@ -627,6 +629,11 @@ __device__ __forceinline__ uint32_t find_job(const PathParams& p, uint32_t x) {
 }
 
 // path.slang:1792-1866 up to integrate: sampler, film-filtered pinhole camera ray.
+// A pixel's samples take neighbouring slots, and so do its later rays (every pass packs its
+// queue in order): the lanes of a warp then read mostly the same nodes and shade the same
+// surfaces.  With a pixel's samples an image apart, whole renders took 3-6% longer (1080p
+// 64 spp flock frame 375.8 vs 365.4 ms, 256x256 16 spp 1.99 vs 1.88 ms, preview batch 34.9 vs
+// 33.8 ms); tiles of 4 or 8 image rows under this order: equal or 1% slower.
 template <bool BATCH>
 __global__ void k_camera(PathParams p) {
     const uint32_t n = p.counters[7];
@@ -635,7 +642,7 @@ __global__ void k_camera(PathParams p) {
         const Job& J = BATCH ? p.jobs[j] : p.job0;
         if (BATCH) p.slot_job[slot] = j;
         uint32_t local = slot - J.slot_base;
-        uint32_t pixel = local % J.npix, sidx = J.wave_first + local / J.npix;
+        uint32_t pixel = local / J.wave_samples, sidx = J.wave_first + local % J.wave_samples;
         uint32_t px = pixel % J.cam.width, py = pixel / J.cam.width;
         uint32_t pseed = screen_ray_hash(px, py, 0u, J.seed);
         uint32_t rng = screen_ray_hash(px, py, sidx, J.seed);
@@ -1205,8 +1212,8 @@ __global__ void __launch_bounds__(SPLIT_BLOCK) k_split(const __grid_constant__ P
         const float4 T = p.thr[slot];
         const uint32_t meta = __float_as_uint(T.w), bounce = meta & 0xffu;
         if (J.primary_ids && bounce == 0u) {
-            const uint32_t local = slot - J.slot_base, pixel = local % J.npix;
-            if (J.wave_first + local / J.npix == J.first_sample) {
+            const uint32_t local = slot - J.slot_base, pixel = local / J.wave_samples;
+            if (J.wave_first + local % J.wave_samples == J.first_sample) {
                 J.primary_ids[2 * pixel] = inst;
                 J.primary_ids[2 * pixel + 1] = hit ? __float_as_uint(__ldg(&J.sv.blas_tris[3u * size_t(__float_as_uint(p.hit[i].w))]).w) : 0xffffffffu;
             }
@@ -1285,7 +1292,7 @@ __global__ void __launch_bounds__(VKB_SHADE_BLOCK, VKB_SHADE_MIN_BLOCKS) k_shade
         float3 thr = f3(T.x, T.y, T.z), rad = f3(R.x, R.y, R.z);
         uint32_t dropped = __float_as_uint(R.w), rng = rg.x, pseed = rg.y;
         uint32_t local = slot - J.slot_base;
-        uint32_t sidx = J.wave_first + local / J.npix;
+        uint32_t sidx = J.wave_first + local % J.wave_samples;
         float limit = bounce == 0 ? J.clamp_direct : J.clamp_indirect;
         uint32_t vtx = bounce;
         float4 sc = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 0));   // path_scatter
@@ -1621,7 +1628,7 @@ __global__ void k_accumulate(PathParams p) {
             // Guide renders: the guides of a dropped sample are zero too (path.slang:1946-1950).
             float4 ga = J.guide_accum[2 * pixel], gn = J.guide_accum[2 * pixel + 1];
             for (uint32_t k = 0; k < J.wave_samples; ++k) {
-                uint32_t slot = J.slot_base + k * J.npix + pixel;
+                uint32_t slot = J.slot_base + pixel * J.wave_samples + k;
                 float4 T = p.thr[slot], R = p.rad[slot];
                 dl += __float_as_uint(R.w);
                 float3 v = f3(R.x, R.y, R.z) * J.env.exposure;
@@ -1636,14 +1643,24 @@ __global__ void k_accumulate(PathParams p) {
             }
             J.guide_accum[2 * pixel] = ga;
             J.guide_accum[2 * pixel + 1] = gn;
-        } else
-        for (uint32_t k = 0; k < J.wave_samples; ++k) {
-            uint32_t slot = J.slot_base + k * J.npix + pixel;
-            float4 T = p.thr[slot], R = p.rad[slot];
-            dl += __float_as_uint(R.w);
-            float3 v = f3(R.x, R.y, R.z) * J.env.exposure;
-            if ((__float_as_uint(T.w) & META_NONFINITE) || !finite3(v)) { v = f3(0.f); dp++; }
-            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += 1.f;
+        } else {
+            // Four samples' loads in flight; the sums stay one at a time in sample order.
+            const uint32_t first = J.slot_base + pixel * J.wave_samples;
+            for (uint32_t k = 0; k < J.wave_samples; k += 4u) {
+                float4 R[4];
+                uint32_t meta[4];
+                #pragma unroll
+                for (uint32_t u = 0; u < 4u; ++u)
+                    if (k + u < J.wave_samples) { R[u] = p.rad[first + k + u]; meta[u] = __float_as_uint(p.thr[first + k + u].w); }
+                #pragma unroll
+                for (uint32_t u = 0; u < 4u; ++u) {
+                    if (k + u >= J.wave_samples) break;
+                    dl += __float_as_uint(R[u].w);
+                    float3 v = f3(R[u].x, R[u].y, R[u].z) * J.env.exposure;
+                    if ((meta[u] & META_NONFINITE) || !finite3(v)) { v = f3(0.f); dp++; }
+                    sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += 1.f;
+                }
+            }
         }
         J.accum[pixel] = sum;
         if (dl) atomicAdd(&p.counters[5], dl);
