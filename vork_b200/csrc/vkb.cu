@@ -194,6 +194,7 @@ std::vector<Bvh4Node> collapse_blas(const std::vector<BvhNode>& n2) {
             todo.push_back({child[k], idx});
             child[k] = idx;
         }
+        node.child2 = node.child;
         out[q] = node;
     }
     return out;

@@ -22,13 +22,17 @@ namespace vkb {
 struct alignas(16) BvhNode { float4 a, b, c; int4 d; };
 
 // Four child boxes of a 4-wide node as planes (component k = child slot k), one 128-byte
-// line per node: plane 2a is the low face of axis a, plane 2a+1 the high face, so a ray
-// reads its near face of axis a at 2a + (direction negative) and its far face at the
-// other.  child = (c0, c1, c2, c3) as in BvhNode; an unused slot has the empty box
-// lo = +inf, hi = -inf, which every ray misses.  Traversal runs on these nodes; they are
-// collapsed from the binary trees (every internal node at even depth takes its children
-// and the children of its internal children).
-struct alignas(16) Bvh4Node { float4 plane[6]; int4 child; int4 pad; };
+// line of four 32-byte sectors: (lo x, lo y), (hi x, hi y), (lo z, children), (hi z,
+// children again).  A ray reads each sector whole: its near x face leads sector
+// (direction x negative), its near z face sector 2 + (direction z negative), and only the
+// two y faces may come the wrong way round.  child = (c0, c1, c2, c3) as in BvhNode; an
+// unused slot has the empty box lo = +inf, hi = -inf, which every ray misses.  The lanes of
+// a warp read different nodes, and the L1 data pipe serves them almost one at a time: it was
+// 86-91% busy on the flock (issue 56-64%) with seven 16-byte loads a visit.  Four 32-byte
+// loads: 1080p 64 spp flock frame 366.3 -> 356.3 ms, small scenes (which hit L1 and are bound
+// by issue) equal to 1% faster.  Traversal runs on these nodes; they are collapsed from the binary trees (every internal node at
+// even depth takes its children and the children of its internal children).
+struct alignas(128) Bvh4Node { float4 lo_x, lo_y, hi_x, hi_y, lo_z; int4 child; float4 hi_z; int4 child2; };
 static_assert(sizeof(Bvh4Node) == 128, "one 128-byte line per 4-wide node");
 
 // Compressed 8-wide BLAS node, 80 bytes (the layout of vkb_host::Wide8Node, built on the
@@ -41,7 +45,7 @@ struct alignas(16) Bvh8Node { float4 h; uint4 b; uint4 q[3]; };
 static_assert(sizeof(Bvh8Node) == 80, "80-byte compressed 8-wide node");
 
 // One TLAS leaf, in Morton order: the instance's world->object rows and what its BLAS needs.
-struct alignas(16) TlasLeaf { float4 w2o[3]; uint32_t instance, node_offset, tri_offset, flags; };
+struct alignas(64) TlasLeaf { float4 w2o[3]; uint32_t instance, node_offset, tri_offset, flags; };
 constexpr uint32_t LEAF_CULL_BACKFACES = 1u;
 
 struct MeshInfo {
@@ -148,6 +152,11 @@ __device__ __forceinline__ void node_boxes(const BvhNode& n, const RaySpace& r, 
     tl = lmin <= lmax * 1.00000024f ? lmin : __int_as_float(0x7f800000);
     tr = rmin <= rmax * 1.00000024f ? rmin : __int_as_float(0x7f800000);
 }
+// Eight floats of one 32-byte sector (read-only data).
+__device__ __forceinline__ void ld8(const void* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(p));
+}
 // Three-input float min / max (sm_100 instructions; no NaN reaches them here).
 __device__ __forceinline__ float max3f(float a, float b, float c) { float r; asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
 __device__ __forceinline__ float min3f(float a, float b, float c) { float r; asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
@@ -237,9 +246,8 @@ struct RayRef {
     const float4* d;
     uint32_t i;
     __device__ __forceinline__ static float3 ld3(const float4* p) {
-        float x, y, z;
-        asm volatile("ld.global.nc.f32 %0, [%3];\n\tld.global.nc.f32 %1, [%3+4];\n\tld.global.nc.f32 %2, [%3+8];"
-                     : "=f"(x), "=f"(y), "=f"(z) : "l"(p));
+        float x, y, z, w;
+        asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x), "=f"(y), "=f"(z), "=f"(w) : "l"(p));
         return f3(x, y, z);
     }
     __device__ __forceinline__ float3 origin() const { return ld3(o + i); }
@@ -352,12 +360,15 @@ struct TraceLane {
             }
         } else {
             if (COUNT) { count->nodes++; if (in_blas) count->blas_nodes++; }
-            const float4* p = reinterpret_cast<const float4*>(nodes + node);
-            const uint32_t sx = __float_as_uint(rs.idir.x) >> 31, sy = __float_as_uint(rs.idir.y) >> 31, sz = __float_as_uint(rs.idir.z) >> 31;
-            const float4 nx = __ldg(p + sx), fx = __ldg(p + (sx ^ 1u));
-            const float4 ny = __ldg(p + 2u + sy), fy = __ldg(p + (3u - sy));
-            const float4 nz = __ldg(p + 4u + sz), fz = __ldg(p + (5u - sz));
-            const int4 ch = __ldg(reinterpret_cast<const int4*>(p + 6));
+            const char* p = reinterpret_cast<const char*>(nodes + node);
+            const uint32_t sx = (__float_as_uint(rs.idir.x) >> 31) << 5, sz = (__float_as_uint(rs.idir.z) >> 31) << 5;
+            float4 nx, fx, ny, fy, nz, fz, c0, c1;
+            ld8(p + sx, nx, ny);
+            ld8(p + (sx ^ 32u), fx, fy);
+            ld8(p + 64u + sz, nz, c0);
+            ld8(p + 64u + (sz ^ 32u), fz, c1);
+            const int4 ch = make_int4(__float_as_int(c0.x), __float_as_int(c0.y), __float_as_int(c0.z), __float_as_int(c0.w));
+            if (int(__float_as_uint(rs.idir.x) ^ __float_as_uint(rs.idir.y)) < 0) { const float4 y = ny; ny = fy; fy = y; }
             uint32_t k0 = slot_key(nx.x, ny.x, nz.x, fx.x, fy.x, fz.x, rs, tbest, 0u);
             uint32_t k1 = slot_key(nx.y, ny.y, nz.y, fx.y, fy.y, fz.y, rs, tbest, 1u);
             uint32_t k2 = slot_key(nx.z, ny.z, nz.z, fx.z, fy.z, fz.z, rs, tbest, 2u);
@@ -422,8 +433,10 @@ struct TraceLane {
             if (++steps >= TRACE_STEP_LIMIT) { fail(err, 2u); return; }
             if (COUNT) count->instances++;
             const TlasLeaf* lf = s.tlas_leaves + (~node);
-            float4 r0 = __ldg(&lf->w2o[0]), r1 = __ldg(&lf->w2o[1]), r2 = __ldg(&lf->w2o[2]);
-            uint4 info = __ldg(reinterpret_cast<const uint4*>(&lf->instance));
+            float4 r0, r1, r2, in;
+            ld8(&lf->w2o[0], r0, r1);
+            ld8(&lf->w2o[2], r2, in);
+            const uint4 info = make_uint4(__float_as_uint(in.x), __float_as_uint(in.y), __float_as_uint(in.z), __float_as_uint(in.w));
             const float3 o = so, d = sd;
             so = f3(r0.x * o.x + r0.y * o.y + r0.z * o.z + r0.w, r1.x * o.x + r1.y * o.y + r1.z * o.z + r1.w, r2.x * o.x + r2.y * o.y + r2.z * o.z + r2.w);
             sd = f3(r0.x * d.x + r0.y * d.y + r0.z * d.z, r1.x * d.x + r1.y * d.y + r1.z * d.z, r2.x * d.x + r2.y * d.y + r2.z * d.z);

@@ -360,9 +360,10 @@ __global__ void k_bvh_parity(uint32_t n_internal, const uint32_t* node_parent, u
 }
 // Child slot k of a 4-wide node: box planes and reference.
 __device__ __host__ __forceinline__ void set_slot(Bvh4Node& q, int k, float lx, float hx, float ly, float hy, float lz, float hz, int ref) {
-    float* pl = reinterpret_cast<float*>(q.plane);
-    pl[0 * 4 + k] = lx; pl[1 * 4 + k] = hx; pl[2 * 4 + k] = ly; pl[3 * 4 + k] = hy; pl[4 * 4 + k] = lz; pl[5 * 4 + k] = hz;
+    auto set = [k](void* plane, float v) { static_cast<float*>(plane)[k] = v; };
+    set(&q.lo_x, lx); set(&q.hi_x, hx); set(&q.lo_y, ly); set(&q.hi_y, hy); set(&q.lo_z, lz); set(&q.hi_z, hz);
     reinterpret_cast<int*>(&q.child)[k] = ref;
+    reinterpret_cast<int*>(&q.child2)[k] = ref;
 }
 // The slots of the 4-wide node for binary node b: each leaf child keeps its slot, each
 // internal child gives its own two children (internal references stay binary indices).
@@ -381,7 +382,6 @@ __device__ __host__ __forceinline__ Bvh4Node collapse_node(const BvhNode* n2, co
         }
     }
     for (; k < 4; ++k) set_slot(q, k, INFINITY, -INFINITY, INFINITY, -INFINITY, INFINITY, -INFINITY, ~0);
-    q.pad = make_int4(0, 0, 0, 0);
     return q;
 }
 // Every even-depth internal node i of the binary tree becomes 4-wide node i (the odd
