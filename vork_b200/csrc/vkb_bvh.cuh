@@ -56,10 +56,10 @@ struct MeshInfo {
 };
 
 #ifndef VKB_SMEM_STACK
-#define VKB_SMEM_STACK 24
+#define VKB_SMEM_STACK 16
 #endif
 #ifndef VKB_SPILL_STACK
-#define VKB_SPILL_STACK 40
+#define VKB_SPILL_STACK 48
 #endif
 // Traversal stacks: the first SMEM_STACK entries live in shared memory as
 // [entry][thread] (lane l of a 128-thread block always touches bank l, whatever depth
@@ -72,9 +72,22 @@ constexpr int STACK_CAP = SMEM_STACK + SPILL_STACK;
 constexpr int SPILL_STACK8 = 104;
 constexpr int STACK_CAP8 = SMEM_STACK + SPILL_STACK8;
 constexpr int TRACE_BLOCK = 128;
+// The ray in world space (origin, direction, their slab terms) is kept there the same way:
+// an instance entry reads the first two and its end the last two, instead of the queue entry
+// again and three reciprocals (sixteen stack entries leave the room: 256x256 16 spp 1.84 ->
+// 1.81 ms, 641x359 std/path 5.00 -> 4.91 ms, flock frame 355.1 -> 354.0 ms; with 24 entries the
+// L1 given up takes half of it back).
+constexpr int WORLD_ORIGIN = 0, WORLD_DIR = 3, WORLD_IDIR = 6, WORLD_OOD = 9, WORLD_FLOATS = 12;
 struct TraceStack {
     int* r;
     int* spill;
+    float* world;
+    __device__ __forceinline__ void keep(int at, float3 v) const {
+        world[at * TRACE_BLOCK] = v.x; world[(at + 1) * TRACE_BLOCK] = v.y; world[(at + 2) * TRACE_BLOCK] = v.z;
+    }
+    __device__ __forceinline__ float3 kept(int at) const {
+        return make_float3(world[at * TRACE_BLOCK], world[(at + 1) * TRACE_BLOCK], world[(at + 2) * TRACE_BLOCK]);
+    }
     __device__ __forceinline__ void put(int i, int v) {
         if (SPILL_STACK == 0 || i < SMEM_STACK) r[i * TRACE_BLOCK] = v;
         else spill[i - SMEM_STACK] = v;
@@ -232,18 +245,12 @@ static_assert(VKB_BLAS_LEAF_MAX >= 1 && VKB_BLAS_LEAF_MAX <= 4, "leaf counts are
 struct HitRecord { float t, u, v; uint32_t tri, inst; };
 
 // A world ray in global memory: entry i of an origin queue and a direction queue (xyz of
-// float4).  Traversal re-reads it when it enters or leaves an instance instead of keeping
-// six registers live across the loop; the volatile loads keep the compiler from caching
-// the values, and the queue bases are the same for every thread (uniform registers).
+// float4), read once, when its traversal starts.
 struct RayRef {
     const float4* o;
     const float4* d;
     uint32_t i;
-    __device__ __forceinline__ static float3 ld3(const float4* p) {
-        float x, y, z, w;
-        asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x), "=f"(y), "=f"(z), "=f"(w) : "l"(p));
-        return f3(x, y, z);
-    }
+    __device__ __forceinline__ static float3 ld3(const float4* p) { const float4 v = __ldg(p); return f3(v.x, v.y, v.z); }
     __device__ __forceinline__ float3 origin() const { return ld3(o + i); }
     __device__ __forceinline__ float3 dir() const { return ld3(d + i); }
 };
@@ -281,8 +288,10 @@ struct TraceLane {
     HitRecord hit;
 
     // Returns false when there is nothing to traverse.
-    __device__ __forceinline__ bool start(const SceneView& s, RayRef ray, float tmax) {
-        make_space(rs, ray.origin(), ray.dir(), false);
+    __device__ __forceinline__ bool start(const SceneView& s, RayRef ray, float tmax, TraceStack stk) {
+        const float3 o = ray.origin(), d = ray.dir();
+        make_space(rs, o, d, false);
+        stk.keep(WORLD_ORIGIN, o); stk.keep(WORLD_DIR, d); stk.keep(WORLD_IDIR, rs.idir); stk.keep(WORLD_OOD, rs.ood);
         tbest = tmax; sp = 0; steps = 0;
         found = false; in_blas = false; cull = false;
         nodes = s.tlas_nodes; tri_base = 0; cur_instance = 0;
@@ -424,7 +433,7 @@ struct TraceLane {
     // A BLAS leaf, the end of an instance, an instance entry: whichever the ray is at, and
     // then those that follow in this order without a node between them, so an instance left
     // for another one sets up the ray's space once.
-    __device__ __forceinline__ void special(const SceneView& s, RayRef ray, uint32_t* err, TraceCount* count, TraceStack stk) {
+    __device__ __forceinline__ void special(const SceneView& s, uint32_t* err, TraceCount* count, TraceStack stk) {
         if (in_blas && node != LEAVE) {
             if (++steps >= TRACE_STEP_LIMIT) { fail(err, 2u); return; }
             // BLAS leaf: up to VKB_BLAS_LEAF_MAX triangles in leaf order, ~((first << 2) | (count - 1)).
@@ -450,31 +459,33 @@ struct TraceLane {
             respace = true;
         }
         if (node == DONE || (!respace && in_blas)) return;
-        float3 so = ray.origin(), sd = ray.dir();
-        if (node < 0) {
-            // Instance entry: the ray in object space.
-            if (++steps >= TRACE_STEP_LIMIT) { fail(err, 2u); return; }
-            if (COUNT) count->instances++;
-            const TlasLeaf* lf = s.tlas_leaves + (~node);
-            float4 r0, r1, r2, in;
-            ld8(&lf->w2o[0], r0, r1);
-            ld8(&lf->w2o[2], r2, in);
-            const uint4 info = make_uint4(__float_as_uint(in.x), __float_as_uint(in.y), __float_as_uint(in.z), __float_as_uint(in.w));
-            const float3 o = so, d = sd;
-            so = f3(r0.x * o.x + r0.y * o.y + r0.z * o.z + r0.w, r1.x * o.x + r1.y * o.y + r1.z * o.z + r1.w, r2.x * o.x + r2.y * o.y + r2.z * o.z + r2.w);
-            sd = f3(r0.x * d.x + r0.y * d.y + r0.z * d.z, r1.x * d.x + r1.y * d.y + r1.z * d.z, r2.x * d.x + r2.y * d.y + r2.z * d.z);
-            cur_instance = info.x;
-            if (W8) nodes8 = s.blas8 + info.y;
-            else nodes = s.blas_nodes + info.y;
-            tri_base = info.z;
-            cull = !ANY && (info.w & LEAF_CULL_BACKFACES);
-            if (sp >= CAP) { fail(err, 1u); return; }
-            stk.put(sp, LEAVE);
-            ++sp;
-            in_blas = true;
-            node = 0;
+        if (node >= 0) {
+            rs.idir = stk.kept(WORLD_IDIR);
+            rs.ood = stk.kept(WORLD_OOD);
+            return;
         }
-        make_space(rs, so, sd, in_blas);
+        // Instance entry: the ray in object space.
+        if (++steps >= TRACE_STEP_LIMIT) { fail(err, 2u); return; }
+        if (COUNT) count->instances++;
+        const TlasLeaf* lf = s.tlas_leaves + (~node);
+        float4 r0, r1, r2, in;
+        ld8(&lf->w2o[0], r0, r1);
+        ld8(&lf->w2o[2], r2, in);
+        const uint4 info = make_uint4(__float_as_uint(in.x), __float_as_uint(in.y), __float_as_uint(in.z), __float_as_uint(in.w));
+        const float3 o = stk.kept(WORLD_ORIGIN), d = stk.kept(WORLD_DIR);
+        const float3 so = f3(r0.x * o.x + r0.y * o.y + r0.z * o.z + r0.w, r1.x * o.x + r1.y * o.y + r1.z * o.z + r1.w, r2.x * o.x + r2.y * o.y + r2.z * o.z + r2.w);
+        const float3 sd = f3(r0.x * d.x + r0.y * d.y + r0.z * d.z, r1.x * d.x + r1.y * d.y + r1.z * d.z, r2.x * d.x + r2.y * d.y + r2.z * d.z);
+        cur_instance = info.x;
+        if (W8) nodes8 = s.blas8 + info.y;
+        else nodes = s.blas_nodes + info.y;
+        tri_base = info.z;
+        cull = !ANY && (info.w & LEAF_CULL_BACKFACES);
+        if (sp >= CAP) { fail(err, 1u); return; }
+        stk.put(sp, LEAVE);
+        ++sp;
+        in_blas = true;
+        node = 0;
+        make_space(rs, so, sd, true);
     }
 };
 
@@ -482,10 +493,10 @@ template <bool ANY, bool COUNT = false, bool W8 = false>
 __device__ __forceinline__ bool trace_ray(const SceneView& s, RayRef ray, float tmax, HitRecord& hit, uint32_t* err,
                                           TraceCount* count, TraceStack stk) {
     TraceLane<ANY, COUNT, W8> L;
-    if (!L.start(s, ray, tmax)) return false;
+    if (!L.start(s, ray, tmax, stk)) return false;
     while (!L.done()) {
         if (L.node >= 0) L.visit(err, count, stk);
-        if (L.at_special()) L.special(s, ray, err, count, stk);
+        if (L.at_special()) L.special(s, err, count, stk);
     }
     hit = L.hit;
     return L.found;

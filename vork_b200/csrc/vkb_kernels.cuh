@@ -688,12 +688,13 @@ __device__ __forceinline__ bool trace_any(const SceneView& sv, RayRef ray, float
                                           TraceStack stk) {
     return trace_ray<ANY, COUNT, W8>(sv, ray, tmax, h, err, tc, stk);
 }
-// This thread's column of the block's shared-memory traversal stack (W8: the deeper local
-// part of the 8-wide BLAS traversal).
+// This thread's column of the block's shared-memory traversal stack and world rays (W8: the
+// deeper local part of the 8-wide BLAS traversal).
 #define VKB_STACK_DECL_W(W8)                                                                             \
     __shared__ int stack_r_[SMEM_STACK * TRACE_BLOCK];                                                  \
+    __shared__ float world_[WORLD_FLOATS * TRACE_BLOCK];                                                \
     int stack_spill_[(W8) ? SPILL_STACK8 : (SPILL_STACK > 0 ? SPILL_STACK : 1)];                         \
-    TraceStack stk{stack_r_ + threadIdx.x, stack_spill_};
+    TraceStack stk{stack_r_ + threadIdx.x, stack_spill_, world_ + threadIdx.x};
 #define VKB_STACK_DECL VKB_STACK_DECL_W(false)
 // Lanes of a warp refill together once at most this many are still tracing.
 #ifndef VKB_TRACE_REFILL
@@ -747,7 +748,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace(Pat
     auto take = [&](uint32_t r) {
         ray = r;
         if (BATCH) job = job_of_slot<true>(p, __float_as_uint(p.ray_d[cur][r].w));
-        L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.ray_o[cur], p.ray_d[cur], r}, p.ray_o[cur][r].w);
+        L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.ray_o[cur], p.ray_d[cur], r}, p.ray_o[cur][r].w, stk);
     };
     const uint32_t share = short_share(n, gridDim.x * (TRACE_BLOCK / 32u));
     if (share) {
@@ -772,7 +773,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace(Pat
             const uint32_t r = base + uint32_t(__popc(idle & ((1u << lane) - 1u)));
             if (L.done() && r < n) take(r);
         }
-        if (L.at_special()) L.special(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.ray_o[cur], p.ray_d[cur], ray}, p.err, &tc, stk);
+        if (L.at_special()) L.special(BATCH ? p.jobs[job].sv : p.job0.sv, p.err, &tc, stk);
         do {
             if (L.node >= 0) L.visit(p.err, &tc, stk);
         } while (__popc(__ballot_sync(0xffffffffu, L.node >= 0)) > VKB_TRACE_NODES);
@@ -799,24 +800,24 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace_sha
     TraceCount tc;
     TraceLane<true, COUNT, W8> L;
     constexpr uint32_t NONE = 0xffffffffu;
-    uint32_t e = NONE, rid = 0, phase = 0, occ = 0, job = 0;
+    uint32_t e = NONE, phase = 0, occ = 0, job = 0;
     // Starts entry e's next ray from phase ph on; false when the entry has no ray left.
     auto begin = [&](uint32_t ph) -> bool {
         const uint32_t flags = __float_as_uint(p.sa_c[e].w);
         if (ph == 0u) {
-            if ((flags & SH_TRACE_A) && L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.sa_o, p.sa_d, e}, p.sa_o[e].w)) { phase = 0u; rid = e; return true; }
+            if ((flags & SH_TRACE_A) && L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.sa_o, p.sa_d, e}, p.sa_o[e].w, stk)) { phase = 0u; return true; }
         }
         if (ph <= 1u && (flags & SH_HAS_B) && (flags & SH_TRACE_B)) {
             const uint32_t slot = __float_as_uint(p.sa_d[e].w);
-            if (L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.sb_o, p.sb_d, slot}, p.sb_o[slot].w)) { phase = 1u; rid = slot; return true; }
+            if (L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.sb_o, p.sb_d, slot}, p.sb_o[slot].w, stk)) { phase = 1u; return true; }
         }
         if constexpr (EXT) {
             const uint32_t slot = __float_as_uint(p.sa_d[e].w);
             if (ph <= 2u && (flags & SH_HAS_C)) {
-                if (L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.sc_o, p.sc_d, slot}, p.sc_o[slot].w)) { phase = 2u; rid = slot; return true; }
+                if (L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.sc_o, p.sc_d, slot}, p.sc_o[slot].w, stk)) { phase = 2u; return true; }
             }
             if (flags & SH_HAS_D) {
-                if (L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.sd_o, p.sd_d, slot}, p.sd_o[slot].w)) { phase = 3u; rid = slot; return true; }
+                if (L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.sd_o, p.sd_d, slot}, p.sd_o[slot].w, stk)) { phase = 3u; return true; }
             }
         }
         return false;
@@ -881,16 +882,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace_sha
                 if (e == NONE && r < n) take(r);
             }
         }
-        if (L.at_special()) {
-            // The traversal re-reads its ray (instance entry, return to world space):
-            // phase 0 the light ray A, 1 the light ray B, 2 the environment ray, 3 the mesh ray.
-            RayRef ray{phase ? p.sb_o : p.sa_o, phase ? p.sb_d : p.sa_d, rid};
-            if constexpr (EXT) {
-                if (phase == 2u) ray = RayRef{p.sc_o, p.sc_d, rid};
-                else if (phase == 3u) ray = RayRef{p.sd_o, p.sd_d, rid};
-            }
-            L.special(BATCH ? p.jobs[job].sv : p.job0.sv, ray, p.err, &tc, stk);
-        }
+        if (L.at_special()) L.special(BATCH ? p.jobs[job].sv : p.job0.sv, p.err, &tc, stk);
         do {
             if (L.node >= 0) L.visit(p.err, &tc, stk);
         } while (__popc(__ballot_sync(0xffffffffu, L.node >= 0)) > VKB_TRACE_NODES);
