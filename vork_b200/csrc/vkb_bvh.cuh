@@ -244,17 +244,6 @@ static_assert(VKB_BLAS_LEAF_MAX >= 1 && VKB_BLAS_LEAF_MAX <= 4, "leaf counts are
 // original id is blas_tris[3 * tri].w), inst: the original instance id.
 struct HitRecord { float t, u, v; uint32_t tri, inst; };
 
-// A world ray in global memory: entry i of an origin queue and a direction queue (xyz of
-// float4), read once, when its traversal starts.
-struct RayRef {
-    const float4* o;
-    const float4* d;
-    uint32_t i;
-    __device__ __forceinline__ static float3 ld3(const float4* p) { const float4 v = __ldg(p); return f3(v.x, v.y, v.z); }
-    __device__ __forceinline__ float3 origin() const { return ld3(o + i); }
-    __device__ __forceinline__ float3 dir() const { return ld3(d + i); }
-};
-
 struct SceneView {
     const Bvh4Node* tlas_nodes;
     const TlasLeaf* tlas_leaves;
@@ -288,8 +277,7 @@ struct TraceLane {
     HitRecord hit;
 
     // Returns false when there is nothing to traverse.
-    __device__ __forceinline__ bool start(const SceneView& s, RayRef ray, float tmax, TraceStack stk) {
-        const float3 o = ray.origin(), d = ray.dir();
+    __device__ __forceinline__ bool start(const SceneView& s, float3 o, float3 d, float tmax, TraceStack stk) {
         make_space(rs, o, d, false);
         stk.keep(WORLD_ORIGIN, o); stk.keep(WORLD_DIR, d); stk.keep(WORLD_IDIR, rs.idir); stk.keep(WORLD_OOD, rs.ood);
         tbest = tmax; sp = 0; steps = 0;
@@ -490,10 +478,10 @@ struct TraceLane {
 };
 
 template <bool ANY, bool COUNT = false, bool W8 = false>
-__device__ __forceinline__ bool trace_ray(const SceneView& s, RayRef ray, float tmax, HitRecord& hit, uint32_t* err,
+__device__ __forceinline__ bool trace_ray(const SceneView& s, float3 o, float3 d, float tmax, HitRecord& hit, uint32_t* err,
                                           TraceCount* count, TraceStack stk) {
     TraceLane<ANY, COUNT, W8> L;
-    if (!L.start(s, ray, tmax, stk)) return false;
+    if (!L.start(s, o, d, tmax, stk)) return false;
     while (!L.done()) {
         if (L.node >= 0) L.visit(err, count, stk);
         if (L.at_special()) L.special(s, err, count, stk);

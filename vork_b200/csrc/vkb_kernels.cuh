@@ -505,7 +505,8 @@ struct PathParams {
     // [0],[1] ray counts, [2] shadow count, [3] ext rays, [4] shadow rays, [5] dropped light,
     // [6] dropped paths, [7] path slots of this wave, [8] pixels of this wave's jobs
     // [9] radiance-cache records of this wave, [10] adaptive pixel-samples skipped,
-    // [11], [12] rays the closest-hit and shadow traces have taken, [13] this bounce's hits
+    // [11], [12] rays the closest-hit and shadow traces have taken, [13] this bounce's hits,
+    // [14] k_paths has taken the wave's remaining bounces
     uint32_t* counters;
     unsigned long long* work;  // instrumented traversal: closest nodes, tris, instances, blas nodes; shadow nodes, tris, blas nodes
     uint32_t* err;
@@ -684,9 +685,8 @@ __device__ __forceinline__ void flush_count(unsigned long long* dst, uint32_t v)
 #define VKB_TRACE_MIN_BLOCKS 8
 #endif
 template <bool ANY, bool COUNT, bool W8 = false>
-__device__ __forceinline__ bool trace_any(const SceneView& sv, RayRef ray, float tmax, HitRecord& h, uint32_t* err, TraceCount* tc,
-                                          TraceStack stk) {
-    return trace_ray<ANY, COUNT, W8>(sv, ray, tmax, h, err, tc, stk);
+__device__ __forceinline__ bool trace_any(const SceneView& sv, float4 o, float4 d, HitRecord& h, uint32_t* err, TraceCount* tc, TraceStack stk) {
+    return trace_ray<ANY, COUNT, W8>(sv, f3(o.x, o.y, o.z), f3(d.x, d.y, d.z), o.w, h, err, tc, stk);
 }
 // This thread's column of the block's shared-memory traversal stack and world rays (W8: the
 // deeper local part of the 8-wide BLAS traversal).
@@ -700,13 +700,25 @@ __device__ __forceinline__ bool trace_any(const SceneView& sv, RayRef ray, float
 #ifndef VKB_TRACE_REFILL
 #define VKB_TRACE_REFILL 20
 #endif
-// A warp keeps visiting nodes while more than this many lanes are at one; then it takes
-// every waiting special step (leaf, instance entry and exit) together.
+// A warp keeps visiting nodes while more than this many lanes are at one (closest hits,
+// shadow rays); then it takes every waiting special step (leaf, instance entry and exit)
+// together.
 #ifndef VKB_TRACE_NODES
-#define VKB_TRACE_NODES 12
+#define VKB_TRACE_NODES 14
+#endif
+#ifndef VKB_SHADOW_NODES
+#define VKB_SHADOW_NODES 12
 #endif
 static_assert(VKB_TRACE_REFILL >= 1 && VKB_TRACE_REFILL <= 31, "refill threshold in lanes");
-static_assert(VKB_TRACE_NODES >= 0 && VKB_TRACE_NODES <= 31, "node threshold in lanes");
+static_assert(VKB_TRACE_NODES >= 0 && VKB_TRACE_NODES <= 31 && VKB_SHADOW_NODES >= 0 && VKB_SHADOW_NODES <= 31, "node thresholds in lanes");
+// One round of a warp's traversals: the special steps that wait, then node visits.
+template <int NODES, class Lane>
+__device__ __forceinline__ void advance(Lane& L, const SceneView& sv, uint32_t* err, TraceCount* tc, TraceStack stk) {
+    if (L.at_special()) L.special(sv, err, tc, stk);
+    do {
+        if (L.node >= 0) L.visit(err, tc, stk);
+    } while (__popc(__ballot_sync(0xffffffffu, L.node >= 0)) > NODES);
+}
 // Lanes of each warp that take an entry when a queue of n entries is shorter than the lanes
 // of `warps` resident warps (0: it is not).  A short queue takes as long as its longest
 // entry, and an entry's steps wait for every branch its warp's other lanes take: n entries
@@ -726,9 +738,10 @@ __device__ __forceinline__ uint32_t share_index(uint32_t share) {
 // visits; at two dozen rays a warp nearly always had one lane at a leaf, an instance entry
 // or exit and one finishing, so with one branch per step every pass paid for all four with
 // a lane or two in each (542 warp instructions per ray on the flock at 480x270).  So
-//  - the specials wait until at most VKB_TRACE_NODES lanes have a node (8 / 10 / 12 / 16 /
-//    20: 403.8 / 401.4 / 400.9 / 403.1 / 413.5 ms for the 1080p 64 spp flock frame; each
-//    ray's own order, and so every hit, is unchanged);
+//  - the specials wait until at most VKB_TRACE_NODES lanes have a node (both traces at 8 /
+//    10 / 12 / 16 / 20: 403.8 / 401.4 / 400.9 / 403.1 / 413.5 ms for the 1080p 64 spp flock frame;
+//    later closest hits at 10 / 12 / 14: 358.2 / 355.6 / 354.5, shadow rays at 8 / 12 / 16: 357.4 /
+//    355.6 / 355.7; each ray's own order, and so every hit, is unchanged);
 //  - results are written, and new rays taken from the queue with one atomic, by all the
 //    warp's idle lanes together once at most VKB_TRACE_REFILL still trace (each lane as soon
 //    as it finishes is slower: that code then runs on single lanes).
@@ -737,7 +750,7 @@ __device__ __forceinline__ uint32_t share_index(uint32_t share) {
 template <bool COUNT, bool BATCH, bool W8 = false>
 __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace(PathParams p, int cur) {
     VKB_STACK_DECL_W(W8)
-    const uint32_t n = p.counters[cur];
+    const uint32_t n = p.counters[14] ? 0u : p.counters[cur];
     if (blockIdx.x == 0 && threadIdx.x == 0) { atomicAdd(&p.counters[3], n); p.counters[13] = 0u; }
     const uint32_t lane = threadIdx.x & 31u;
     TraceCount tc;
@@ -747,8 +760,9 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace(Pat
     bool drained = false;
     auto take = [&](uint32_t r) {
         ray = r;
-        if (BATCH) job = job_of_slot<true>(p, __float_as_uint(p.ray_d[cur][r].w));
-        L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.ray_o[cur], p.ray_d[cur], r}, p.ray_o[cur][r].w, stk);
+        const float4 o = __ldg(&p.ray_o[cur][r]), d = __ldg(&p.ray_d[cur][r]);
+        if (BATCH) job = job_of_slot<true>(p, __float_as_uint(d.w));
+        L.start(BATCH ? p.jobs[job].sv : p.job0.sv, f3(o.x, o.y, o.z), f3(d.x, d.y, d.z), o.w, stk);
     };
     const uint32_t share = short_share(n, gridDim.x * (TRACE_BLOCK / 32u));
     if (share) {
@@ -773,10 +787,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace(Pat
             const uint32_t r = base + uint32_t(__popc(idle & ((1u << lane) - 1u)));
             if (L.done() && r < n) take(r);
         }
-        if (L.at_special()) L.special(BATCH ? p.jobs[job].sv : p.job0.sv, p.err, &tc, stk);
-        do {
-            if (L.node >= 0) L.visit(p.err, &tc, stk);
-        } while (__popc(__ballot_sync(0xffffffffu, L.node >= 0)) > VKB_TRACE_NODES);
+        advance<VKB_TRACE_NODES>(L, BATCH ? p.jobs[job].sv : p.job0.sv, p.err, &tc, stk);
     }
     if (COUNT) {
         flush_count(&p.work[0], tc.nodes);
@@ -786,43 +797,42 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace(Pat
     }
 }
 
-// Shadow entries with lane refill (as k_trace): a lane carries one entry through its
-// ray A, then its ray B (the second estimator's, when present and traced), then adds
-// the unoccluded contributions to the slot's radiance.
-// EXT: waves with an image environment or emissive meshes, whose entries may carry an
-// environment ray (phase 2) and a mesh ray (phase 3) after the light rays A and B.
-template <bool COUNT, bool BATCH, bool EXT, bool W8 = false>
-__global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace_shadow(PathParams p) {
-    VKB_STACK_DECL_W(W8)
-    const uint32_t n = p.counters[2];
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&p.counters[4], n);
-    const uint32_t lane = threadIdx.x & 31u;
-    TraceCount tc;
+// A shadow entry's way through its rays: the light ray A (phase 0), the second estimator's
+// light ray B (1, when present and traced), in EXT waves an environment ray (2) and a mesh
+// ray (3); then the unoccluded contributions join the slot's radiance.
+// OWN: the entry was written by this thread in this kernel (no read-only loads).
+template <bool COUNT, bool BATCH, bool EXT, bool W8, bool OWN = false>
+struct ShadowLane {
+    __device__ __forceinline__ static float4 ray4(const float4* v) { return OWN ? *v : __ldg(v); }
+    static constexpr uint32_t NONE = 0xffffffffu;
     TraceLane<true, COUNT, W8> L;
-    constexpr uint32_t NONE = 0xffffffffu;
     uint32_t e = NONE, phase = 0, occ = 0, job = 0;
-    // Starts entry e's next ray from phase ph on; false when the entry has no ray left.
-    auto begin = [&](uint32_t ph) -> bool {
+    __device__ __forceinline__ bool start(const PathParams& p, uint32_t ph, float4 o, float4 d, TraceStack stk) {
+        phase = ph;
+        return L.start(BATCH ? p.jobs[job].sv : p.job0.sv, f3(o.x, o.y, o.z), f3(d.x, d.y, d.z), o.w, stk);
+    }
+    // Starts the entry's next ray from phase ph on; false when it has no ray left.
+    __device__ __forceinline__ bool begin(const PathParams& p, uint32_t ph, TraceStack stk) {
         const uint32_t flags = __float_as_uint(p.sa_c[e].w);
         if (ph == 0u) {
-            if ((flags & SH_TRACE_A) && L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.sa_o, p.sa_d, e}, p.sa_o[e].w, stk)) { phase = 0u; return true; }
+            if ((flags & SH_TRACE_A) && start(p, 0u, ray4(&p.sa_o[e]), ray4(&p.sa_d[e]), stk)) return true;
         }
         if (ph <= 1u && (flags & SH_HAS_B) && (flags & SH_TRACE_B)) {
             const uint32_t slot = __float_as_uint(p.sa_d[e].w);
-            if (L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.sb_o, p.sb_d, slot}, p.sb_o[slot].w, stk)) { phase = 1u; return true; }
+            if (start(p, 1u, ray4(&p.sb_o[slot]), ray4(&p.sb_d[slot]), stk)) return true;
         }
         if constexpr (EXT) {
             const uint32_t slot = __float_as_uint(p.sa_d[e].w);
             if (ph <= 2u && (flags & SH_HAS_C)) {
-                if (L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.sc_o, p.sc_d, slot}, p.sc_o[slot].w, stk)) { phase = 2u; return true; }
+                if (start(p, 2u, ray4(&p.sc_o[slot]), ray4(&p.sc_d[slot]), stk)) return true;
             }
             if (flags & SH_HAS_D) {
-                if (L.start(BATCH ? p.jobs[job].sv : p.job0.sv, RayRef{p.sd_o, p.sd_d, slot}, p.sd_o[slot].w, stk)) { phase = 3u; return true; }
+                if (start(p, 3u, ray4(&p.sd_o[slot]), ray4(&p.sd_d[slot]), stk)) return true;
             }
         }
         return false;
-    };
-    auto finish = [&]() {
+    }
+    __device__ __forceinline__ void finish(const PathParams& p) {
         const float4 sc = p.sa_c[e];
         const uint32_t slot = __float_as_uint(p.sa_d[e].w), flags = __float_as_uint(sc.w);
         float3 total = (occ & 1u) ? f3(0.f) : f3(sc.x, sc.y, sc.z);
@@ -848,29 +858,44 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace_sha
         }
         p.rad[slot] = make_float4(r.x + add.x, r.y + add.y, r.z + add.z, __uint_as_float(dropped));
         e = NONE;
-    };
-    auto take = [&](uint32_t r) {
-        e = r;
+    }
+    __device__ __forceinline__ void take(const PathParams& p, uint32_t entry, TraceStack stk) {
+        e = entry;
         occ = 0u;
-        if (BATCH) job = job_of_slot<true>(p, __float_as_uint(p.sa_d[r].w));
-        if (!begin(0u)) finish();
-    };
+        if (BATCH) job = job_of_slot<true>(p, __float_as_uint(p.sa_d[entry].w));
+        if (!begin(p, 0u, stk)) finish(p);
+    }
+    // After a ray's end: the entry's next ray, or the entry's.
+    __device__ __forceinline__ void next(const PathParams& p, TraceStack stk) {
+        if (L.found) occ |= 1u << phase;
+        if constexpr (EXT) { if (phase == 3u || !begin(p, phase + 1u, stk)) finish(p); }
+        else { if (phase != 0u || !begin(p, 1u, stk)) finish(p); }
+    }
+};
+
+// Shadow entries with lane refill (as k_trace): a lane carries one entry to its end.
+// EXT: waves with an image environment or emissive meshes.
+template <bool COUNT, bool BATCH, bool EXT, bool W8 = false>
+__global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace_shadow(PathParams p) {
+    VKB_STACK_DECL_W(W8)
+    const uint32_t n = p.counters[2];
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&p.counters[4], n);
+    const uint32_t lane = threadIdx.x & 31u;
+    TraceCount tc;
+    constexpr uint32_t NONE = 0xffffffffu;
+    ShadowLane<COUNT, BATCH, EXT, W8> S;
     bool drained = false;
     const uint32_t share = short_share(n, gridDim.x * (TRACE_BLOCK / 32u));
     if (share) {
         const uint32_t r = share_index(share);
-        if (lane < share && r < n) take(r);
+        if (lane < share && r < n) S.take(p, r, stk);
         drained = true;
     }
     for (;;) {
-        uint32_t act = __ballot_sync(0xffffffffu, !L.done());
+        uint32_t act = __ballot_sync(0xffffffffu, !S.L.done());
         if (act == 0u || (!drained && uint32_t(__popc(act)) <= uint32_t(VKB_TRACE_REFILL))) {
-            if (e != NONE && L.done()) {
-                if (L.found) occ |= 1u << phase;
-                if constexpr (EXT) { if (phase == 3u || !begin(phase + 1u)) finish(); }
-                else { if (phase != 0u || !begin(1u)) finish(); }
-            }
-            const uint32_t idle = __ballot_sync(0xffffffffu, e == NONE);
+            if (S.e != NONE && S.L.done()) S.next(p, stk);
+            const uint32_t idle = __ballot_sync(0xffffffffu, S.e == NONE);
             if (drained) {
                 if (idle == 0xffffffffu) break;
             } else {
@@ -879,13 +904,10 @@ __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace_sha
                 base = __shfl_sync(0xffffffffu, base, 0);
                 drained = base + uint32_t(__popc(idle)) >= n;
                 const uint32_t r = base + uint32_t(__popc(idle & ((1u << lane) - 1u)));
-                if (e == NONE && r < n) take(r);
+                if (S.e == NONE && r < n) S.take(p, r, stk);
             }
         }
-        if (L.at_special()) L.special(BATCH ? p.jobs[job].sv : p.job0.sv, p.err, &tc, stk);
-        do {
-            if (L.node >= 0) L.visit(p.err, &tc, stk);
-        } while (__popc(__ballot_sync(0xffffffffu, L.node >= 0)) > VKB_TRACE_NODES);
+        advance<VKB_SHADOW_NODES>(S.L, BATCH ? p.jobs[S.job].sv : p.job0.sv, p.err, &tc, stk);
     }
     if (COUNT) {
         flush_count(&p.work[3], tc.nodes);
@@ -1157,6 +1179,43 @@ __device__ __noinline__ void cache_append(const PathParams& p, float3 world, flo
     }
 }
 
+// The camera hit's instance and original triangle (leaf-order triangle tri; inst ~0u: none).
+__device__ __forceinline__ void store_ids(const Job& J, uint32_t slot, uint32_t inst, uint32_t tri) {
+    const uint32_t local = slot - J.slot_base, pixel = local / J.wave_samples;
+    if (J.wave_first + local % J.wave_samples != J.first_sample) return;
+    J.primary_ids[2 * pixel] = inst;
+    J.primary_ids[2 * pixel + 1] = inst != 0xffffffffu ? __float_as_uint(__ldg(&J.sv.blas_tris[3u * size_t(tri)]).w) : 0xffffffffu;
+}
+// A ray that left the scene (path.slang:1484-1512): the constant world light or the image,
+// and camera-visible suns; the path ends.
+template <bool EXT>
+__device__ __forceinline__ void finish_miss(const PathParams& p, const Job& J, uint32_t slot, float3 dir, float4 T, uint32_t bounce) {
+    const uint32_t ray_event = bounce == 0 ? VKB_RAY_CAMERA : ((__float_as_uint(T.w) >> 24) & 0x3fu);
+    const float limit = bounce == 0 ? J.clamp_direct : J.clamp_indirect;
+    const float4 R = p.rad[slot];
+    const float3 thr = f3(T.x, T.y, T.z);
+    float3 rad = f3(R.x, R.y, R.z);
+    uint32_t dropped = __float_as_uint(R.w);
+    float3 sky;
+    if (ray_event == VKB_RAY_CAMERA && !J.env.camera_sees_environment) sky = get3(J.env.background);
+    else {
+        sky = EXT ? env_radiance(J, dir) : get3(J.env.radiance);
+        if (ray_event == VKB_RAY_CAMERA)
+            for (uint32_t l = 0; l < J.num_lights; ++l) {
+                const vkb_light& L = J.lights[l];
+                if (L.position[3] != 0.f || !(L.shadow_offsets[0] & VKB_RAY_CAMERA)) continue;
+                sky = sky + emitter_eval(L, f3(0.f), dir).radiance;
+            }
+    }
+    if (EXT && J.env_w && bounce > 0u) {
+        // path.slang:1463: an escape after a BSDF sample, weighed against the
+        // environment strategy.
+        const float prev = p.prev[slot].w;
+        if (prev > 0.f) sky = sky * mis_power(prev, env_density(J, dir));
+    }
+    rad = rad + clamp_sample(thr * sky, limit, dropped);
+    p.rad[slot] = make_float4(rad.x, rad.y, rad.z, __uint_as_float(dropped));
+}
 // Before a bounce's shade pass: the rays that left the scene add what they see and end
 // here; the hits' queue indices are packed, a block's in order, into the bounce's spent
 // origin queue (nothing reads the origins after the trace), counted in counters[13].
@@ -1169,11 +1228,12 @@ __device__ __noinline__ void cache_append(const PathParams& p, float3 world, flo
 // The bounce's queue counters are reset here too: no kernel reads them between their last
 // reader and this one.
 constexpr int SPLIT_BLOCK = 512;
+constexpr int PATHS_BLOCKS = 2;   // blocks of k_paths per SM
 template <bool BATCH, bool EXT>
 __global__ void __launch_bounds__(SPLIT_BLOCK) k_split(const __grid_constant__ PathParams p, int cur) {
     __shared__ uint32_t warp_hits[SPLIT_BLOCK / 32], base;
     if (blockIdx.x == 0 && threadIdx.x == 0) { p.counters[cur ^ 1] = 0u; p.counters[2] = 0u; p.counters[11] = 0u; p.counters[12] = 0u; }
-    const uint32_t n = p.counters[cur], lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t n = p.counters[14] ? 0u : p.counters[cur], lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     uint32_t* hits = reinterpret_cast<uint32_t*>(p.ray_o[cur]);
     for (uint32_t first = blockIdx.x * SPLIT_BLOCK; first < n; first += gridDim.x * SPLIT_BLOCK) {
         const uint32_t i = first + threadIdx.x;
@@ -1202,45 +1262,254 @@ __global__ void __launch_bounds__(SPLIT_BLOCK) k_split(const __grid_constant__ P
         const uint32_t slot = __float_as_uint(rd.w);
         const Job& J = BATCH ? p.jobs[job_of_slot<true>(p, slot)] : p.job0;
         const float4 T = p.thr[slot];
-        const uint32_t meta = __float_as_uint(T.w), bounce = meta & 0xffu;
-        if (J.primary_ids && bounce == 0u) {
-            const uint32_t local = slot - J.slot_base, pixel = local / J.wave_samples;
-            if (J.wave_first + local % J.wave_samples == J.first_sample) {
-                J.primary_ids[2 * pixel] = inst;
-                J.primary_ids[2 * pixel + 1] = hit ? __float_as_uint(__ldg(&J.sv.blas_tris[3u * size_t(__float_as_uint(p.hit[i].w))]).w) : 0xffffffffu;
-            }
-        }
+        const uint32_t bounce = __float_as_uint(T.w) & 0xffu;
+        if (J.primary_ids && bounce == 0u) store_ids(J, slot, inst, hit ? __float_as_uint(p.hit[i].w) : 0u);
         if (hit) continue;
-        // Miss: path.slang:1484-1512 with the constant world light and camera-visible suns.
-        const uint32_t ray_event = bounce == 0 ? VKB_RAY_CAMERA : ((meta >> 24) & 0x3fu);
-        const float limit = bounce == 0 ? J.clamp_direct : J.clamp_indirect;
-        const float4 R = p.rad[slot];
-        const float3 dir = f3(rd.x, rd.y, rd.z), thr = f3(T.x, T.y, T.z);
-        float3 rad = f3(R.x, R.y, R.z);
-        uint32_t dropped = __float_as_uint(R.w);
-        float3 sky;
-        if (ray_event == VKB_RAY_CAMERA && !J.env.camera_sees_environment) sky = get3(J.env.background);
-        else {
-            sky = EXT ? env_radiance(J, dir) : get3(J.env.radiance);
-            if (ray_event == VKB_RAY_CAMERA)
-                for (uint32_t l = 0; l < J.num_lights; ++l) {
-                    const vkb_light& L = J.lights[l];
-                    if (L.position[3] != 0.f || !(L.shadow_offsets[0] & VKB_RAY_CAMERA)) continue;
-                    sky = sky + emitter_eval(L, f3(0.f), dir).radiance;
-                }
-        }
-        if (EXT && J.env_w && bounce > 0u) {
-            // path.slang:1463: an escape after a BSDF sample, weighed against the
-            // environment strategy.
-            const float prev = p.prev[slot].w;
-            if (prev > 0.f) sky = sky * mis_power(prev, env_density(J, dir));
-        }
-        rad = rad + clamp_sample(thr * sky, limit, dropped);
-        p.rad[slot] = make_float4(rad.x, rad.y, rad.z, __uint_as_float(dropped));
+        finish_miss<EXT>(p, J, slot, f3(rd.x, rd.y, rd.z), T, bounce);
     }
 }
 
-// integrate's per-vertex body (path.slang:1340-1709) for one queued extension hit.
+// integrate's per-vertex body (path.slang:1340-1709) for one extension hit (hh, inst) of the
+// path in a slot.  out.shadow_entry() gives the place of its shadow entry, out.next_ray()
+// takes its next extension ray.
+template <bool EXT, class Out>
+__device__ __forceinline__ void shade_vertex(const PathParams& p, const Job& J, uint32_t slot, float3 dir, float4 hh, uint32_t inst, Out& out) {
+    float4 T = p.thr[slot], R = p.rad[slot];
+    uint2 rg = p.rng[slot];
+    uint32_t meta = __float_as_uint(T.w);
+    uint32_t bounce = meta & 0xffu, diffuse = (meta >> 8) & 0xffu, glossy = (meta >> 16) & 0xffu;
+    float3 thr = f3(T.x, T.y, T.z), rad = f3(R.x, R.y, R.z);
+    uint32_t dropped = __float_as_uint(R.w), rng = rg.x, pseed = rg.y;
+    uint32_t local = slot - J.slot_base;
+    uint32_t sidx = J.wave_first + local % J.wave_samples;
+    float limit = bounce == 0 ? J.clamp_direct : J.clamp_indirect;
+    uint32_t vtx = bounce;
+    float4 sc = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 0));   // path_scatter
+    Surface s = hit_surface(J, inst, __float_as_uint(hh.w), hh.y, hh.z, dir);
+    const vkb_material& mt = J.materials[__ldg(&J.inst_info[inst]).y];
+    Closure c;
+    c.base_color = get3(mt.base_color); c.base_weight = mt.base_weight; c.base_metalness = mt.base_metalness;
+    c.specular_color = get3(mt.specular_color); c.specular_weight = mt.specular_weight;
+    c.specular_roughness = mt.specular_roughness; c.specular_ior = mt.specular_ior; c.optical_ior = 0.f;
+    c.n = s.geometric;
+    boundary_closure_air(c);
+    float3 view = -dir;
+    if (EXT && mt.emission_luminance > 0.f && ((mt.flags & 2u) || s.entering)) {
+        // Surface emission (path.slang:1580-1591) on the side the material covers,
+        // weighed against the mesh strategy after a BSDF sample.
+        const float3 emitted = get3(mt.emission_color) * mt.emission_luminance;
+        float mis = 1.f;
+        if (bounce > 0u && J.em_tris) {
+            const float4 pv = p.prev[slot];
+            if (pv.w > 0.f) {
+                const uint32_t tri = __float_as_uint(hh.w);
+                const float4* tp = J.sv.blas_tris + 3u * size_t(tri);
+                const float4 q0 = __ldg(tp), q1 = __ldg(tp + 1), q2 = __ldg(tp + 2);
+                const float4 M[3] = {__ldg(&J.o2w[3 * inst]), __ldg(&J.o2w[3 * inst + 1]), __ldg(&J.o2w[3 * inst + 2])};
+                const float3 e1 = mvec(M, f3(q1.x - q0.x, q1.y - q0.y, q1.z - q0.z)), e2 = mvec(M, f3(q2.x - q0.x, q2.y - q0.y, q2.z - q0.z));
+                const float area = length(cross(e1, e2)) * 0.5f;
+                mis = mis_power(pv.w, mesh_pdf(J, inst, __float_as_uint(q0.w), area, f3(pv.x, pv.y, pv.z), s.world, s.face));
+            }
+        }
+        rad = rad + clamp_sample(thr * emitted * mis, limit, dropped);
+    }
+    // Radiance cache: record this vertex, and at the query vertex stop the path
+    // here (the query kernel adds thr x the cached outgoing radiance).
+    const bool cache_query = p.cache.mode == 1u && bounce >= p.cache.vertex;
+    if (cache_query || (p.cache.mode == 2u && bounce >= 1u)) cache_append(p, s.world, view, s.geometric, c.specular_roughness, c.base_metalness, c.base_color, slot, bounce, thr, rad);
+    if (!cache_query) {
+    float3 iface = dot(s.geometric, view) > 0.f ? s.geometric : s.face;
+    Prepared pr = transport_prepare(p.lut, c, view, s.geometric, iface);
+    BsdfSample smp = transport_sample(c, view, sc.x, sc.y, sc.z, pr);
+    if (!finite3(smp.dir) || !finite3(smp.weight) || !isfinite(smp.pdf)) {
+        meta |= META_NONFINITE;
+    } else {
+        // The image-environment and mesh strategies first: their shadow rays go
+        // to the slot's own buffers at once, so nothing of theirs stays live
+        // across the analytic estimate (the sample groups and the order of the
+        // sums in the shadow kernel do not depend on this order).
+        // environment_next_event (path.slang:1096-1120): a proposal direction,
+        // the diffuse and specular responses MIS-weighted against continuing
+        // there (continuation_mask, path.slang:1003-1010), one visibility ray
+        // to infinity; clamped on its own.
+        bool trace_c = false, trace_d = false;
+        uint32_t cont = 0u;
+        if (EXT && bounce < J.bounces[0]) {
+            if (diffuse < J.bounces[1]) cont |= VKB_RAY_DIFFUSE;
+            if (glossy < J.bounces[2] && (diffuse == 0u || (J.caustics & 1u))) cont |= VKB_RAY_SPECULAR;
+        }
+        if (EXT && J.env_w) {
+            const float4 eu = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 3));   // path_environment
+            float epdf = 0.f;
+            const float3 edir = env_sample(J, eu.x, eu.y, epdf);
+            float3 ev = f3(0.f);
+            if (epdf > 0.f) {
+                const float3 emitted = env_radiance(J, edir);
+                if (maxc(emitted) > 0.f) {
+                    #pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const uint32_t event = k == 0 ? VKB_RAY_DIFFUSE : VKB_RAY_SPECULAR;
+                        if (!event_hemisphere(event, edir, s.face, s.geometric)) continue;
+                        const float3 response = eval_mask(c, view, edir, event, pr);
+                        if (maxc(response) <= 0.f) continue;
+                        const float bpdf = (cont & event) ? pdf_mask(c, view, edir, event, pr) : 0.f;
+                        ev = ev + emitted * response * (mis_power(epdf, bpdf) / epdf);
+                    }
+                }
+            }
+            if (any_nonzero(ev)) {
+                const float3 oc = path_origin(s, edir), cc = thr * ev;
+                p.sc_o[slot] = make_float4(oc.x, oc.y, oc.z, FP32_MAX);
+                p.sc_d[slot] = make_float4(edir.x, edir.y, edir.z, 0.f);
+                p.sc_c[slot] = make_float4(cc.x, cc.y, cc.z, 0.f);
+                trace_c = true;
+            }
+        }
+        if (EXT && J.em_tris) {
+            // mesh_next_event (path.slang:1121-1167), constant emission: a point on a
+            // source triangle, the diffuse and specular responses MIS-weighted against
+            // continuing there, one visibility ray between the offset end points.
+            const float4 g = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 2));   // path_triangle
+            uint32_t ei, ep; float b1, b2;
+            if (em_sample(J, g.z, g.x, g.y, ei, ep, b1, b2)) {
+                const EmGeometry eg = em_geometry(J, ei, ep, b1, b2);
+                const float3 delta = eg.point - s.world;
+                const float distance = length(delta);
+                if (distance > 0.f) {
+                    const float3 axis = delta / distance;
+                    const float mpdf = mesh_pdf(J, ei, ep, eg.area, s.world, eg.point, eg.face);
+                    const vkb_material& em = J.materials[__ldg(&J.inst_info[ei]).y];
+                    const bool front = dot(eg.face, axis) < 0.f;
+                    const float3 emitted = get3(em.emission_color) * em.emission_luminance;
+                    if (mpdf > 0.f && ((em.flags & 2u) || front) && maxc(emitted) > 0.f) {
+                        const float3 start = path_origin(s, axis);
+                        const float3 end = surface_ray_origin(eg.point, eg.error, front ? eg.face : -eg.face, -axis);
+                        const float3 connection = end - start;
+                        const float extent = length(connection);
+                        float3 response = f3(0.f);
+                        if (extent > 0.f) {
+                            #pragma unroll
+                            for (int k = 0; k < 2; ++k) {
+                                const uint32_t event = k == 0 ? VKB_RAY_DIFFUSE : VKB_RAY_SPECULAR;
+                                if (!event_hemisphere(event, axis, s.face, s.geometric)) continue;
+                                const float3 f = eval_mask(c, view, axis, event, pr);
+                                if (maxc(f) <= 0.f) continue;
+                                const float bpdf = (cont & event) ? pdf_mask(c, view, axis, event, pr) : 0.f;
+                                response = response + f * mis_power(mpdf, bpdf);
+                            }
+                        }
+                        if (any_nonzero(response)) {
+                            const float3 md = thr * (response * emitted / mpdf), cdir = connection / extent;
+                            p.sd_o[slot] = make_float4(start.x, start.y, start.z, extent);
+                            p.sd_d[slot] = make_float4(cdir.x, cdir.y, cdir.z, 0.f);
+                            p.sd_c[slot] = make_float4(md.x, md.y, md.z, 0.f);
+                            trace_d = true;
+                        }
+                    }
+                }
+            }
+        }
+        // next_event (path.slang:851-951): one analytic light, two estimators.
+        float3 va = f3(0.f), vb = f3(0.f);
+        bool trace_a = false, has_b = false, trace_b = false;
+        float3 oa, da, ob, db; float la = 0.f, lb = 0.f;
+        if (J.num_lights > 0) {
+            float4 u = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 1));   // path_light
+            float probability;
+            uint32_t li = tree_pick(J.tree, J.tree_nodes, s.world, u.z, u.w, probability);
+            if (probability > 0.f && li < J.num_lights) {
+                const vkb_light& L = J.lights[li];
+                uint32_t contribution = L.shadow_offsets[VKB_LIGHT_CONTRIBUTION_WORD];
+                bool shadowed = (L.shadow_offsets[VKB_LIGHT_RAY_WORD] & VKB_LIGHT_RAY_SHADOWED) != 0u;
+                if ((contribution & VKB_LIGHT_LINK_ALL) || L.shadow_offsets[VKB_LIGHT_LINK_WORD]) {
+                    LightSample src = emitter_sample(L, s.world, u.x, u.y);
+                    float3 power = src.delta ? src.radiance : (src.pdf > 0.f ? src.radiance / src.pdf : f3(0.f));
+                    va = analytic_mis_response(c, view, src.dir, s.face, contribution, src.pdf, pr) * power / probability;
+                    va = light_threshold(va, J.light_threshold, rng);
+                    if (any_nonzero(va) && shadowed) {
+                        oa = path_origin(s, src.dir);
+                        ray_connection(oa, s.world, src.dir, src.distance, da, la);
+                        trace_a = true;
+                    }
+                    bool continuation = (contribution & smp.event) && event_hemisphere(smp.event, smp.dir, s.face, s.geometric);
+                    if (continuation && dot(smp.dir, smp.dir) > 0.f) {
+                        EmitterEval e = emitter_eval(L, s.world, smp.dir);
+                        if (e.pdf > 0.f) {
+                            float w = smp.pdf > 0.f ? mis_power(smp.pdf, e.pdf) : 1.f;
+                            vb = light_threshold(smp.weight * e.radiance * (w / probability), J.light_threshold, rng);
+                            if (any_nonzero(vb)) {
+                                has_b = true;
+                                if (shadowed) {
+                                    ob = path_origin(s, smp.dir);
+                                    ray_connection(ob, s.world, smp.dir, e.distance, db, lb);
+                                    trace_b = true;
+                                }
+                            }
+                        }
+                    }
+                }
+            }
+        }
+        float3 ca = thr * va, cb = thr * vb;
+        if (trace_a || trace_b || trace_c || trace_d) {
+            uint32_t flags = (trace_a ? SH_TRACE_A : 0u) | (has_b ? SH_HAS_B : 0u) | (trace_b ? SH_TRACE_B : 0u) | (bounce == 0 ? SH_DIRECT : 0u) |
+                             (trace_c ? SH_HAS_C : 0u) | (trace_d ? SH_HAS_D : 0u);
+            const uint32_t si = out.shadow_entry();
+            p.sa_o[si] = trace_a ? make_float4(oa.x, oa.y, oa.z, la) : make_float4(0.f, 0.f, 0.f, 0.f);
+            p.sa_d[si] = make_float4(da.x, da.y, da.z, __uint_as_float(slot));
+            p.sa_c[si] = make_float4(ca.x, ca.y, ca.z, __uint_as_float(flags));
+            if (has_b) {
+                p.sb_c[slot] = make_float4(cb.x, cb.y, cb.z, 0.f);
+                if (trace_b) { p.sb_o[slot] = make_float4(ob.x, ob.y, ob.z, lb); p.sb_d[slot] = make_float4(db.x, db.y, db.z, 0.f); }
+            }
+        } else {
+            rad = rad + clamp_sample(ca + cb, limit, dropped);
+        }
+        // Continuation (path.slang:1683-1708).
+        bool go = bounce < J.bounces[0];
+        uint32_t event = smp.event;
+        if (go) {
+            if (event == VKB_RAY_DIFFUSE) { if (diffuse++ >= J.bounces[1]) go = false; }
+            else if (event == VKB_RAY_SPECULAR) { if (glossy++ >= J.bounces[2] || (diffuse > 0 && !(J.caustics & 1u))) go = false; }
+            else go = false;
+        }
+        if (go && !event_hemisphere(event, smp.dir, s.face, s.geometric)) go = false;
+        if (go) {
+            thr = thr * smp.weight;
+            if (!finite3(thr)) { meta |= META_NONFINITE; go = false; }
+            else if (maxc(thr) <= 0.f) go = false;
+        }
+        if (go && bounce >= ROULETTE_START) {
+            float survive = clampf(maxc(thr), ROULETTE_MIN, ROULETTE_MAX);
+            float4 dec = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 4));
+            if (dec.z > survive) go = false;
+            else thr = thr / survive;
+        }
+        if (go) {
+            float3 o = path_origin(s, smp.dir);
+            if (EXT) p.prev[slot] = make_float4(s.world.x, s.world.y, s.world.z, smp.pdf);
+            out.next_ray(o, smp.dir, slot);
+            meta = (meta & META_NONFINITE) | ((bounce + 1u) & 0xffu) | ((diffuse & 0xffu) << 8) | ((glossy & 0xffu) << 16) | ((event & 0x3fu) << 24);
+        }
+    }
+    }  // !cache_query
+
+    p.thr[slot] = make_float4(thr.x, thr.y, thr.z, __uint_as_float(meta));
+    p.rad[slot] = make_float4(rad.x, rad.y, rad.z, __uint_as_float(dropped));
+    p.rng[slot] = make_uint2(rng, pseed);
+}
+// Shade output of a wavefront pass: the bounce's queues.
+struct QueueOut {
+    const PathParams& p;
+    int nxt;
+    __device__ __forceinline__ uint32_t shadow_entry() const { return group_append(&p.counters[2]); }
+    __device__ __forceinline__ void next_ray(float3 o, float3 d, uint32_t slot) const {
+        const uint32_t ri = group_append(&p.counters[nxt]);
+        p.ray_o[nxt][ri] = make_float4(o.x, o.y, o.z, FP32_MAX);
+        p.ray_d[nxt][ri] = make_float4(d.x, d.y, d.z, __uint_as_float(slot));
+    }
+};
+// A bounce's packed hits.
 // The parameter block is __grid_constant__: `J = p.job0` then refers to it in place
 // (a plain by-value parameter that is referenced gets copied to a 736-byte local frame
 // per thread); one block of 512 per SM (128 registers, a small spill) measured faster
@@ -1261,7 +1530,7 @@ constexpr int SHADE_BLOCK = VKB_SHADE_BLOCK;
 // resident: the blocks that run at once; a short hit list is spread over their warps.
 template <bool BATCH, bool EXT>
 __global__ void __launch_bounds__(VKB_SHADE_BLOCK, VKB_SHADE_MIN_BLOCKS) k_shade(const __grid_constant__ PathParams p, int cur, uint32_t resident) {
-    const int nxt = cur ^ 1;
+    QueueOut out{p, cur ^ 1};
     const uint32_t n = p.counters[13];
     const uint32_t* hits = reinterpret_cast<const uint32_t*>(p.ray_o[cur]);
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
@@ -1274,234 +1543,84 @@ __global__ void __launch_bounds__(VKB_SHADE_BLOCK, VKB_SHADE_MIN_BLOCKS) k_shade
         const float4 rd = p.ray_d[cur][i];
         const uint32_t slot = __float_as_uint(rd.w);
         const Job& J = BATCH ? p.jobs[job_of_slot<true>(p, slot)] : p.job0;
-        const float3 dir = f3(rd.x, rd.y, rd.z);
-        const float4 hh = p.hit[i];
-        const uint32_t inst = p.hit_inst[i];
-        float4 T = p.thr[slot], R = p.rad[slot];
-        uint2 rg = p.rng[slot];
-        uint32_t meta = __float_as_uint(T.w);
-        uint32_t bounce = meta & 0xffu, diffuse = (meta >> 8) & 0xffu, glossy = (meta >> 16) & 0xffu;
-        float3 thr = f3(T.x, T.y, T.z), rad = f3(R.x, R.y, R.z);
-        uint32_t dropped = __float_as_uint(R.w), rng = rg.x, pseed = rg.y;
-        uint32_t local = slot - J.slot_base;
-        uint32_t sidx = J.wave_first + local % J.wave_samples;
-        float limit = bounce == 0 ? J.clamp_direct : J.clamp_indirect;
-        uint32_t vtx = bounce;
-        float4 sc = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 0));   // path_scatter
-        Surface s = hit_surface(J, inst, __float_as_uint(hh.w), hh.y, hh.z, dir);
-        const vkb_material& mt = J.materials[__ldg(&J.inst_info[inst]).y];
-        Closure c;
-        c.base_color = get3(mt.base_color); c.base_weight = mt.base_weight; c.base_metalness = mt.base_metalness;
-        c.specular_color = get3(mt.specular_color); c.specular_weight = mt.specular_weight;
-        c.specular_roughness = mt.specular_roughness; c.specular_ior = mt.specular_ior; c.optical_ior = 0.f;
-        c.n = s.geometric;
-        boundary_closure_air(c);
-        float3 view = -dir;
-        if (EXT && mt.emission_luminance > 0.f && ((mt.flags & 2u) || s.entering)) {
-            // Surface emission (path.slang:1580-1591) on the side the material covers,
-            // weighed against the mesh strategy after a BSDF sample.
-            const float3 emitted = get3(mt.emission_color) * mt.emission_luminance;
-            float mis = 1.f;
-            if (bounce > 0u && J.em_tris) {
-                const float4 pv = p.prev[slot];
-                if (pv.w > 0.f) {
-                    const uint32_t tri = __float_as_uint(hh.w);
-                    const float4* tp = J.sv.blas_tris + 3u * size_t(tri);
-                    const float4 q0 = __ldg(tp), q1 = __ldg(tp + 1), q2 = __ldg(tp + 2);
-                    const float4 M[3] = {__ldg(&J.o2w[3 * inst]), __ldg(&J.o2w[3 * inst + 1]), __ldg(&J.o2w[3 * inst + 2])};
-                    const float3 e1 = mvec(M, f3(q1.x - q0.x, q1.y - q0.y, q1.z - q0.z)), e2 = mvec(M, f3(q2.x - q0.x, q2.y - q0.y, q2.z - q0.z));
-                    const float area = length(cross(e1, e2)) * 0.5f;
-                    mis = mis_power(pv.w, mesh_pdf(J, inst, __float_as_uint(q0.w), area, f3(pv.x, pv.y, pv.z), s.world, s.face));
-                }
-            }
-            rad = rad + clamp_sample(thr * emitted * mis, limit, dropped);
+        shade_vertex<EXT>(p, J, slot, f3(rd.x, rd.y, rd.z), p.hit[i], p.hit_inst[i], out);
+    }
+}
+// Shade output of a path that a lane carries from end to end.
+struct LaneOut {
+    uint32_t i;
+    float3 o, d;
+    bool shadow = false, ray = false;
+    __device__ __forceinline__ uint32_t shadow_entry() { shadow = true; return i; }
+    __device__ __forceinline__ void next_ray(float3 no, float3 nd, uint32_t) { o = no; d = nd; ray = true; }
+};
+// The rest of a small wave in one launch: each warp carries its share of bounce `first`'s
+// rays through every bounce left (closest hit, shade, shadow rays), with the wavefront's own
+// functions on the slot's own records, so every sample's bits are the wavefront's.
+// Bound by latency: a bounce of few rays takes its four launches ~130 us (its longest ray,
+// shade and shadow ray, one after another, whatever the rest do), and here a path waits only
+// for its own warp.  At two blocks per SM nothing spills (204 registers); at four (128
+// registers, 556 B) a 128x128 1 spp render took 368 instead of 343 us, and 487 us in the
+// wavefront.  With more rays than lanes it leaves the bounce to the wavefront's kernels
+// (which pack and refill: 65,536 paths in full warps took 1.25 ms here, 1.0 ms there); when
+// it takes it, counters[14] tells this bounce's kernels that the queue is empty.
+template <bool EXT, bool W8>
+__global__ void __launch_bounds__(TRACE_BLOCK, PATHS_BLOCKS) k_paths(const __grid_constant__ PathParams p, uint32_t first, uint32_t bounces, uint32_t most) {
+    VKB_STACK_DECL_W(W8)
+    const int cur = int(first & 1u);
+    const uint32_t n = p.counters[cur], lane = threadIdx.x & 31u;
+    const uint32_t share = short_share(n, gridDim.x * (TRACE_BLOCK / 32u)), i = share_index(share);
+    if (share == 0u || n > most) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) p.counters[14] = 1u;
+    const Job& J = p.job0;
+    bool alive = lane < share && i < n;
+    uint32_t slot = 0, rays = 0, entries = 0;
+    LaneOut out;
+    out.i = i;
+    float tmax = FP32_MAX;
+    if (alive) {
+        const float4 o = p.ray_o[cur][i], d = p.ray_d[cur][i];
+        out.o = f3(o.x, o.y, o.z); out.d = f3(d.x, d.y, d.z); tmax = o.w;
+        slot = __float_as_uint(d.w);
+    }
+    for (uint32_t b = first; b <= bounces && __any_sync(0xffffffffu, alive); ++b) {
+        float4 hh = make_float4(-1.f, 0.f, 0.f, 0.f);
+        uint32_t inst = 0xffffffffu;
+        {
+            TraceLane<false, false, W8> L;
+            if (alive) { L.start(J.sv, out.o, out.d, tmax, stk); ++rays; }
+            while (__any_sync(0xffffffffu, !L.done())) advance<VKB_TRACE_NODES>(L, J.sv, p.err, nullptr, stk);
+            if (alive && L.found) { hh = make_float4(L.hit.t, L.hit.u, L.hit.v, __uint_as_float(L.hit.tri)); inst = L.hit.inst; }
         }
-        // Radiance cache: record this vertex, and at the query vertex stop the path
-        // here (the query kernel adds thr x the cached outgoing radiance).
-        const bool cache_query = p.cache.mode == 1u && bounce >= p.cache.vertex;
-        if (cache_query || (p.cache.mode == 2u && bounce >= 1u)) cache_append(p, s.world, view, s.geometric, c.specular_roughness, c.base_metalness, c.base_color, slot, bounce, thr, rad);
-        if (!cache_query) {
-        float3 iface = dot(s.geometric, view) > 0.f ? s.geometric : s.face;
-        Prepared pr = transport_prepare(p.lut, c, view, s.geometric, iface);
-        BsdfSample smp = transport_sample(c, view, sc.x, sc.y, sc.z, pr);
-        if (!finite3(smp.dir) || !finite3(smp.weight) || !isfinite(smp.pdf)) {
-            meta |= META_NONFINITE;
-        } else {
-            // The image-environment and mesh strategies first: their shadow rays go
-            // to the slot's own buffers at once, so nothing of theirs stays live
-            // across the analytic estimate (the sample groups and the order of the
-            // sums in the shadow kernel do not depend on this order).
-            // environment_next_event (path.slang:1096-1120): a proposal direction,
-            // the diffuse and specular responses MIS-weighted against continuing
-            // there (continuation_mask, path.slang:1003-1010), one visibility ray
-            // to infinity; clamped on its own.
-            bool trace_c = false, trace_d = false;
-            uint32_t cont = 0u;
-            if (EXT && bounce < J.bounces[0]) {
-                if (diffuse < J.bounces[1]) cont |= VKB_RAY_DIFFUSE;
-                if (glossy < J.bounces[2] && (diffuse == 0u || (J.caustics & 1u))) cont |= VKB_RAY_SPECULAR;
-            }
-            if (EXT && J.env_w) {
-                const float4 eu = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 3));   // path_environment
-                float epdf = 0.f;
-                const float3 edir = env_sample(J, eu.x, eu.y, epdf);
-                float3 ev = f3(0.f);
-                if (epdf > 0.f) {
-                    const float3 emitted = env_radiance(J, edir);
-                    if (maxc(emitted) > 0.f) {
-                        #pragma unroll
-                        for (int k = 0; k < 2; ++k) {
-                            const uint32_t event = k == 0 ? VKB_RAY_DIFFUSE : VKB_RAY_SPECULAR;
-                            if (!event_hemisphere(event, edir, s.face, s.geometric)) continue;
-                            const float3 response = eval_mask(c, view, edir, event, pr);
-                            if (maxc(response) <= 0.f) continue;
-                            const float bpdf = (cont & event) ? pdf_mask(c, view, edir, event, pr) : 0.f;
-                            ev = ev + emitted * response * (mis_power(epdf, bpdf) / epdf);
-                        }
-                    }
-                }
-                if (any_nonzero(ev)) {
-                    const float3 oc = path_origin(s, edir), cc = thr * ev;
-                    p.sc_o[slot] = make_float4(oc.x, oc.y, oc.z, FP32_MAX);
-                    p.sc_d[slot] = make_float4(edir.x, edir.y, edir.z, 0.f);
-                    p.sc_c[slot] = make_float4(cc.x, cc.y, cc.z, 0.f);
-                    trace_c = true;
-                }
-            }
-            if (EXT && J.em_tris) {
-                // mesh_next_event (path.slang:1121-1167), constant emission: a point on a
-                // source triangle, the diffuse and specular responses MIS-weighted against
-                // continuing there, one visibility ray between the offset end points.
-                const float4 g = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 2));   // path_triangle
-                uint32_t ei, ep; float b1, b2;
-                if (em_sample(J, g.z, g.x, g.y, ei, ep, b1, b2)) {
-                    const EmGeometry eg = em_geometry(J, ei, ep, b1, b2);
-                    const float3 delta = eg.point - s.world;
-                    const float distance = length(delta);
-                    if (distance > 0.f) {
-                        const float3 axis = delta / distance;
-                        const float mpdf = mesh_pdf(J, ei, ep, eg.area, s.world, eg.point, eg.face);
-                        const vkb_material& em = J.materials[__ldg(&J.inst_info[ei]).y];
-                        const bool front = dot(eg.face, axis) < 0.f;
-                        const float3 emitted = get3(em.emission_color) * em.emission_luminance;
-                        if (mpdf > 0.f && ((em.flags & 2u) || front) && maxc(emitted) > 0.f) {
-                            const float3 start = path_origin(s, axis);
-                            const float3 end = surface_ray_origin(eg.point, eg.error, front ? eg.face : -eg.face, -axis);
-                            const float3 connection = end - start;
-                            const float extent = length(connection);
-                            float3 response = f3(0.f);
-                            if (extent > 0.f) {
-                                #pragma unroll
-                                for (int k = 0; k < 2; ++k) {
-                                    const uint32_t event = k == 0 ? VKB_RAY_DIFFUSE : VKB_RAY_SPECULAR;
-                                    if (!event_hemisphere(event, axis, s.face, s.geometric)) continue;
-                                    const float3 f = eval_mask(c, view, axis, event, pr);
-                                    if (maxc(f) <= 0.f) continue;
-                                    const float bpdf = (cont & event) ? pdf_mask(c, view, axis, event, pr) : 0.f;
-                                    response = response + f * mis_power(mpdf, bpdf);
-                                }
-                            }
-                            if (any_nonzero(response)) {
-                                const float3 md = thr * (response * emitted / mpdf), cdir = connection / extent;
-                                p.sd_o[slot] = make_float4(start.x, start.y, start.z, extent);
-                                p.sd_d[slot] = make_float4(cdir.x, cdir.y, cdir.z, 0.f);
-                                p.sd_c[slot] = make_float4(md.x, md.y, md.z, 0.f);
-                                trace_d = true;
-                            }
-                        }
-                    }
-                }
-            }
-            // next_event (path.slang:851-951): one analytic light, two estimators.
-            float3 va = f3(0.f), vb = f3(0.f);
-            bool trace_a = false, has_b = false, trace_b = false;
-            float3 oa, da, ob, db; float la = 0.f, lb = 0.f;
-            if (J.num_lights > 0) {
-                float4 u = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 1));   // path_light
-                float probability;
-                uint32_t li = tree_pick(J.tree, J.tree_nodes, s.world, u.z, u.w, probability);
-                if (probability > 0.f && li < J.num_lights) {
-                    const vkb_light& L = J.lights[li];
-                    uint32_t contribution = L.shadow_offsets[VKB_LIGHT_CONTRIBUTION_WORD];
-                    bool shadowed = (L.shadow_offsets[VKB_LIGHT_RAY_WORD] & VKB_LIGHT_RAY_SHADOWED) != 0u;
-                    if ((contribution & VKB_LIGHT_LINK_ALL) || L.shadow_offsets[VKB_LIGHT_LINK_WORD]) {
-                        LightSample src = emitter_sample(L, s.world, u.x, u.y);
-                        float3 power = src.delta ? src.radiance : (src.pdf > 0.f ? src.radiance / src.pdf : f3(0.f));
-                        va = analytic_mis_response(c, view, src.dir, s.face, contribution, src.pdf, pr) * power / probability;
-                        va = light_threshold(va, J.light_threshold, rng);
-                        if (any_nonzero(va) && shadowed) {
-                            oa = path_origin(s, src.dir);
-                            ray_connection(oa, s.world, src.dir, src.distance, da, la);
-                            trace_a = true;
-                        }
-                        bool continuation = (contribution & smp.event) && event_hemisphere(smp.event, smp.dir, s.face, s.geometric);
-                        if (continuation && dot(smp.dir, smp.dir) > 0.f) {
-                            EmitterEval e = emitter_eval(L, s.world, smp.dir);
-                            if (e.pdf > 0.f) {
-                                float w = smp.pdf > 0.f ? mis_power(smp.pdf, e.pdf) : 1.f;
-                                vb = light_threshold(smp.weight * e.radiance * (w / probability), J.light_threshold, rng);
-                                if (any_nonzero(vb)) {
-                                    has_b = true;
-                                    if (shadowed) {
-                                        ob = path_origin(s, smp.dir);
-                                        ray_connection(ob, s.world, smp.dir, e.distance, db, lb);
-                                        trace_b = true;
-                                    }
-                                }
-                            }
-                        }
-                    }
-                }
-            }
-            float3 ca = thr * va, cb = thr * vb;
-            if (trace_a || trace_b || trace_c || trace_d) {
-                uint32_t flags = (trace_a ? SH_TRACE_A : 0u) | (has_b ? SH_HAS_B : 0u) | (trace_b ? SH_TRACE_B : 0u) | (bounce == 0 ? SH_DIRECT : 0u) |
-                                 (trace_c ? SH_HAS_C : 0u) | (trace_d ? SH_HAS_D : 0u);
-                const uint32_t si = group_append(&p.counters[2]);
-                p.sa_o[si] = trace_a ? make_float4(oa.x, oa.y, oa.z, la) : make_float4(0.f, 0.f, 0.f, 0.f);
-                p.sa_d[si] = make_float4(da.x, da.y, da.z, __uint_as_float(slot));
-                p.sa_c[si] = make_float4(ca.x, ca.y, ca.z, __uint_as_float(flags));
-                if (has_b) {
-                    p.sb_c[slot] = make_float4(cb.x, cb.y, cb.z, 0.f);
-                    if (trace_b) { p.sb_o[slot] = make_float4(ob.x, ob.y, ob.z, lb); p.sb_d[slot] = make_float4(db.x, db.y, db.z, 0.f); }
-                }
+        out.shadow = out.ray = false;
+        if (alive) {
+            if (J.primary_ids && b == 0u) store_ids(J, slot, inst, __float_as_uint(hh.w));
+            if (inst == 0xffffffffu) {
+                const float4 T = p.thr[slot];
+                finish_miss<EXT>(p, J, slot, out.d, T, __float_as_uint(T.w) & 0xffu);
             } else {
-                rad = rad + clamp_sample(ca + cb, limit, dropped);
-            }
-            // Continuation (path.slang:1683-1708).
-            bool go = bounce < J.bounces[0];
-            uint32_t event = smp.event;
-            if (go) {
-                if (event == VKB_RAY_DIFFUSE) { if (diffuse++ >= J.bounces[1]) go = false; }
-                else if (event == VKB_RAY_SPECULAR) { if (glossy++ >= J.bounces[2] || (diffuse > 0 && !(J.caustics & 1u))) go = false; }
-                else go = false;
-            }
-            if (go && !event_hemisphere(event, smp.dir, s.face, s.geometric)) go = false;
-            if (go) {
-                thr = thr * smp.weight;
-                if (!finite3(thr)) { meta |= META_NONFINITE; go = false; }
-                else if (maxc(thr) <= 0.f) go = false;
-            }
-            if (go && bounce >= ROULETTE_START) {
-                float survive = clampf(maxc(thr), ROULETTE_MIN, ROULETTE_MAX);
-                float4 dec = sample_group(pseed, sidx, J.sample_mask, vertex_group(vtx, 4));
-                if (dec.z > survive) go = false;
-                else thr = thr / survive;
-            }
-            if (go) {
-                float3 o = path_origin(s, smp.dir);
-                if (EXT) p.prev[slot] = make_float4(s.world.x, s.world.y, s.world.z, smp.pdf);
-                const uint32_t ri = group_append(&p.counters[nxt]);
-                p.ray_o[nxt][ri] = make_float4(o.x, o.y, o.z, FP32_MAX);
-                p.ray_d[nxt][ri] = make_float4(smp.dir.x, smp.dir.y, smp.dir.z, __uint_as_float(slot));
-                meta = (meta & META_NONFINITE) | ((bounce + 1u) & 0xffu) | ((diffuse & 0xffu) << 8) | ((glossy & 0xffu) << 16) | ((event & 0x3fu) << 24);
+                shade_vertex<EXT>(p, J, slot, out.d, hh, inst, out);
             }
         }
-        }  // !cache_query
-    
-        p.thr[slot] = make_float4(thr.x, thr.y, thr.z, __uint_as_float(meta));
-        p.rad[slot] = make_float4(rad.x, rad.y, rad.z, __uint_as_float(dropped));
-        p.rng[slot] = make_uint2(rng, pseed);
+        if (__any_sync(0xffffffffu, out.shadow)) {
+            ShadowLane<false, false, EXT, W8, true> S;
+            if (out.shadow) { S.take(p, i, stk); ++entries; }
+            for (;;) {
+                while (__any_sync(0xffffffffu, !S.L.done())) advance<VKB_SHADOW_NODES>(S.L, J.sv, p.err, nullptr, stk);
+                if (S.e != 0xffffffffu) S.next(p, stk);
+                if (!__any_sync(0xffffffffu, S.e != 0xffffffffu)) break;
+            }
+        }
+        alive = out.ray;
+        tmax = FP32_MAX;
+    }
+    for (int off = 16; off > 0; off >>= 1) {
+        rays += __shfl_xor_sync(0xffffffffu, rays, off);
+        entries += __shfl_xor_sync(0xffffffffu, entries, off);
+    }
+    if (lane == 0u) {
+        if (rays) atomicAdd(&p.counters[3], rays);
+        if (entries) atomicAdd(&p.counters[4], entries);
     }
 }
 // Seed the first ray queue's count from the wave's path-slot count.
@@ -1510,6 +1629,7 @@ __global__ void k_start_wave(uint32_t* counters, uint32_t append_camera) {
     counters[9] = 0u;
     counters[11] = 0u;   // trace fetch counters (closest, shadow)
     counters[12] = 0u;
+    counters[14] = 0u;
 }
 // Adaptive sampling, before the wave of sample index i = wave_first (path.slang:1797-1835):
 // reset at i = 0; from the minimum on a pixel is settled when every channel's standard
@@ -1690,7 +1810,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK) k_debug_trace(SceneView sv, uint3
     VKB_STACK_DECL_W(W8)
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         HitRecord h;
-        bool f = trace_any<false, false, W8>(sv, RayRef{rays, rays + n, i}, rays[i].w, h, err, nullptr, stk);
+        bool f = trace_any<false, false, W8>(sv, rays[i], rays[n + i], h, err, nullptr, stk);
         t[i] = f ? h.t : -1.f;
         ids[2 * i] = f ? h.inst : 0xffffffffu; ids[2 * i + 1] = f ? __float_as_uint(__ldg(&sv.blas_tris[3u * size_t(h.tri)]).w) : 0xffffffffu;
         uv[2 * i] = f ? h.u : 0.f; uv[2 * i + 1] = f ? h.v : 0.f;
@@ -1703,7 +1823,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK) k_debug_occluded(SceneView sv, ui
     VKB_STACK_DECL_W(W8)
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         HitRecord h;
-        occluded[i] = trace_any<true, false, W8>(sv, RayRef{rays, rays + n, i}, rays[i].w, h, err, nullptr, stk) ? 1u : 0u;
+        occluded[i] = trace_any<true, false, W8>(sv, rays[i], rays[n + i], h, err, nullptr, stk) ? 1u : 0u;
     }
 }
 
