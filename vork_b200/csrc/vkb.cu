@@ -53,19 +53,91 @@ struct Unsupported { std::string msg; };
 struct InternalError { std::string msg; };
 struct DeviceTimeout { std::string msg; };
 
+// Device buffers that scenes and calls of one context gave back, for the next ones: an
+// install takes some forty buffers and a display call three, and cudaMalloc / cudaFree (which
+// waits for the device) took most of a small scene's install (20,000 birds on the GPU
+// builders, first frame of 640x360: 14-25 ms from process to process, 4.3 ms with kept
+// buffers).  Bounded; a buffer comes back only when no work on any stream still uses it; what
+// is idle is freed when the context closes or when any allocation runs out of memory.
+class DevicePool {
+public:
+    static constexpr size_t KEEP = size_t(256) << 20;   // idle bytes at most
+    DevicePool() { std::lock_guard<std::mutex> g(all_mutex()); all().push_back(this); }
+    ~DevicePool() {
+        { std::lock_guard<std::mutex> g(all_mutex()); all().erase(std::remove(all().begin(), all().end(), this), all().end()); }
+        trim();
+    }
+    // An idle buffer of at least `bytes` (not twice that and more), or null; bytes: its size.
+    void* take(size_t& bytes) {
+        std::lock_guard<std::mutex> g(m_);
+        auto it = idle_.lower_bound(bytes);
+        if (it == idle_.end() || it->first > 2 * bytes + (size_t(64) << 10)) return nullptr;
+        void* p = it->second;
+        bytes = it->first;
+        held_ -= bytes;
+        idle_.erase(it);
+        return p;
+    }
+    // False when it would hold too much: the caller frees it.
+    bool give(void* p, size_t bytes) {
+        std::lock_guard<std::mutex> g(m_);
+        if (held_ + bytes > KEEP) return false;
+        idle_.emplace(bytes, p);
+        held_ += bytes;
+        return true;
+    }
+    void trim() {
+        std::lock_guard<std::mutex> g(m_);
+        for (auto& b : idle_) cudaFree(b.second);
+        idle_.clear();
+        held_ = 0;
+    }
+    static void trim_all() {
+        std::lock_guard<std::mutex> g(all_mutex());
+        for (DevicePool* p : all()) p->trim();
+    }
+
+private:
+    static std::mutex& all_mutex() { static std::mutex m; return m; }
+    static std::vector<DevicePool*>& all() { static std::vector<DevicePool*> v; return v; }
+    std::mutex m_;
+    std::multimap<size_t, void*> idle_;
+    size_t held_ = 0;
+};
+
 template <class T> struct DBuf {
     T* p = nullptr;
     size_t n = 0;
+    size_t bytes = 0;             // of the allocation
+    DevicePool* pool = nullptr;   // where release() gives it back (none: freed)
+    // Growing frees the old buffer rather than giving it back: queued work may still read it.
     void alloc(size_t count) {
         if (count <= n && p) return;
-        release();
+        if (p) cudaFree(p);
+        p = nullptr; n = 0;
         if (count == 0) return;
-        VKB_CUDA(cudaMalloc(&p, count * sizeof(T)));
+        bytes = count * sizeof(T);
+        void* q = pool ? pool->take(bytes) : nullptr;
+        if (!q) {
+            cudaError_t e = cudaMalloc(&q, bytes);
+            if (e == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                DevicePool::trim_all();
+                e = cudaMalloc(&q, bytes);
+            }
+            if (e != cudaSuccess) throw CudaError{e, "cudaMalloc(&q, bytes)"};
+        }
+        p = static_cast<T*>(q);
         n = count;
     }
-    void release() { if (p) cudaFree(p); p = nullptr; n = 0; }
+    // No work on any stream may still use it.
+    void release() {
+        if (p && !(pool && pool->give(p, bytes))) cudaFree(p);
+        p = nullptr; n = 0;
+    }
     void upload(const T* src, size_t count, cudaStream_t s) { alloc(count); if (count) VKB_CUDA(cudaMemcpyAsync(p, src, count * sizeof(T), cudaMemcpyHostToDevice, s)); }
 };
+template <class... B> void use_pool(DevicePool* pool, B&... bufs) { ((bufs.pool = pool), ...); }
 
 int grid_for(uint32_t n, int block, int sm_count, int per_sm = 8) {
     int need = int((uint64_t(n) + block - 1) / block);
@@ -353,6 +425,7 @@ struct GraphEntry { uint64_t key; cudaGraphExec_t exec; };
 constexpr size_t SINGLE_JOB_WAVE_SLOTS = size_t(64) << 20;   // 14.8 GB of queues per wavefront when full
 struct vkb_ctx {
     int device = 0;
+    DevicePool pool;                    // buffers of closed scenes and finished display calls
     int sms = 148;
     cudaStream_t stream = nullptr;
     DBuf<ushort4> lut;
@@ -429,6 +502,16 @@ struct vkb_scene {
     DBuf<uint2> em_sources;
     DBuf<float> em_tree;
     uint32_t em_count = 0, em_tris = 0, em_leaves = 0;
+
+    explicit vkb_scene(vkb_ctx* c) : ctx(c) {
+        DevicePool* pl = &c->pool;
+        use_pool(pl, o2w_next, changed, vpos, vnrm, blas_tris, tri_nrm, o2w, w2o, inst_lo, inst_hi, tri_lo, tri_hi, indices, tlas_codes, tlas_order,
+                 tlas_leaf_parent, tlas_node_parent, tlas_counters, inst_info, meshes, tlas_nodes, blas4, tlas4, blas8, tlas_odd, tlas_leaves,
+                 d_materials, d_lights, tree, env_img, env_dist, em_inst_source, em_sources, em_tree);
+        use_pool(pl, scratch.codes, scratch.codes_sorted, scratch.ids, scratch.ids_sorted, scratch.leaf_parent, scratch.node_parent,
+                 scratch.counters, scratch.bounds, scratch.cub_temp);
+        use_pool(pl, ploc.clo, ploc.chi, ploc.clo2, ploc.chi2, ploc.nn, ploc.counts, ploc.flags, ploc.offs, ploc.cub_temp);
+    }
 };
 
 namespace {
@@ -1404,6 +1487,7 @@ void build_blas_gpu(vkb_scene* s, uint32_t builder, cudaStream_t st) {
     DBuf<BvhNode> bin;
     DBuf<uint8_t> odd;
     DBuf<uint32_t> leaf_parent, node_parent, counters;
+    use_pool(&s->ctx->pool, bin, odd, leaf_parent, node_parent, counters);
     bin.alloc(max_tris); odd.alloc(max_tris);
     if (builder == VKB_BLAS_BUILD_PLOC) { leaf_parent.alloc(max_tris); node_parent.alloc(max_tris); counters.alloc(max_tris); }
     // Every scratch buffer at the largest mesh's size before the first launch: growing one
@@ -1444,8 +1528,7 @@ void build_blas_gpu(vkb_scene* s, uint32_t builder, cudaStream_t st) {
 vkb_status vkb_scene_create(vkb_ctx* ctx, const vkb_scene_desc* d, vkb_scene** out) {
     if (!ctx || !out) return fail(VKB_INVALID_ARG, "null context or output pointer");
     *out = nullptr;
-    vkb_scene* s = new vkb_scene();
-    s->ctx = ctx;
+    vkb_scene* s = new vkb_scene(ctx);
     const auto t_start = std::chrono::steady_clock::now();
     double blas_host = 0.0;
     vkb_status st = guarded([&] {
@@ -1627,8 +1710,7 @@ vkb_status vkb_scene_fork(vkb_scene* b, vkb_scene** out) {
     if (!b || !out) return fail(VKB_INVALID_ARG, "null scene or output pointer");
     if (b->base) return fail(VKB_INVALID_ARG, "fork of a fork: fork the base scene");
     *out = nullptr;
-    vkb_scene* s = new vkb_scene();
-    s->ctx = b->ctx;
+    vkb_scene* s = new vkb_scene(b->ctx);
     const auto t_start = std::chrono::steady_clock::now();
     vkb_status st = guarded([&] {
         VKB_CUDA(cudaSetDevice(b->ctx->device));
@@ -1923,9 +2005,18 @@ vkb_status vkb_display(vkb_ctx* c, const vkb_display_params* prm, const float* r
         const size_t n = size_t(width) * height;
         if (n == 0) return;
         const size_t out_bytes = n * (prm->bits / 8u) * 4u;
-        DBuf<float4> in;
-        DBuf<unsigned char> o;
-        DBuf<uint32_t> flag;
+        // Kept buffers, given back on every way out once the stream is done with them.
+        struct Work {
+            cudaStream_t s;
+            DBuf<float4> in;
+            DBuf<unsigned char> o;
+            DBuf<uint32_t> flag;
+            ~Work() { cudaStreamSynchronize(s); in.release(); o.release(); flag.release(); }
+        } work{s, {}, {}, {}};
+        DBuf<float4>& in = work.in;
+        DBuf<unsigned char>& o = work.o;
+        DBuf<uint32_t>& flag = work.flag;
+        use_pool(&c->pool, in, o, flag);
         const float4* src = reinterpret_cast<const float4*>(rgba);
         if (!rgba_on_device) { in.upload(reinterpret_cast<const float4*>(rgba), n, s); src = in.p; }
         void* dst = out;
