@@ -872,7 +872,7 @@ struct WaveGrids {
     WaveGrids(const vkb_ctx* c, uint32_t paths) {
         const uint32_t sms = uint32_t(c->sms);
         trace = int(std::max(1u, std::min((paths + 15u) / 16u, sms * VKB_TRACE_MIN_BLOCKS)));
-        split = int(std::max(1u, std::min((paths + SPLIT_BLOCK - 1u) / SPLIT_BLOCK, sms * 16u)));
+        split = int(std::max(1u, std::min((paths + SPLIT_BLOCK * SPLIT_EACH - 1u) / (SPLIT_BLOCK * SPLIT_EACH), sms * 16u)));
         shade = int(std::max(std::min((paths + 63u) / 64u, sms), std::min((paths + SHADE_BLOCK - 1u) / SHADE_BLOCK, sms * uint32_t(c->trace_blocks_per_sm))));
     }
 };

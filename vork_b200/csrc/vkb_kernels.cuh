@@ -1189,10 +1189,9 @@ __device__ __forceinline__ void store_ids(const Job& J, uint32_t slot, uint32_t 
 // A ray that left the scene (path.slang:1484-1512): the constant world light or the image,
 // and camera-visible suns; the path ends.
 template <bool EXT>
-__device__ __forceinline__ void finish_miss(const PathParams& p, const Job& J, uint32_t slot, float3 dir, float4 T, uint32_t bounce) {
+__device__ __forceinline__ void finish_miss(const PathParams& p, const Job& J, uint32_t slot, float3 dir, float4 T, float4 R, uint32_t bounce) {
     const uint32_t ray_event = bounce == 0 ? VKB_RAY_CAMERA : ((__float_as_uint(T.w) >> 24) & 0x3fu);
     const float limit = bounce == 0 ? J.clamp_direct : J.clamp_indirect;
-    const float4 R = p.rad[slot];
     const float3 thr = f3(T.x, T.y, T.z);
     float3 rad = f3(R.x, R.y, R.z);
     uint32_t dropped = __float_as_uint(R.w);
@@ -1219,53 +1218,71 @@ __device__ __forceinline__ void finish_miss(const PathParams& p, const Job& J, u
 // Before a bounce's shade pass: the rays that left the scene add what they see and end
 // here; the hits' queue indices are packed, a block's in order, into the bounce's spent
 // origin queue (nothing reads the origins after the trace), counted in counters[13].
-// Bound by the latency of the queue reads (18% issue).  With the misses in the shade kernel
+// Bound by the latency of the queue and path-state reads: two entries a thread, both entries'
+// reads issued before the block counts its hits (one entry, and the state only of misses and
+// after the count: preview batch 20.6 vs 20.1 ms, flock frame 355.3 vs 352.9 ms).  With the misses in the shade kernel
 // a shade warp ran its long hit path for the few of its lanes that hit: 19, 8 and 11 of 32 at
 // bounces 0, 1, 2 of a 256x256 16 spp still, 23 and 6 in a batch of 24 previews, and each
 // warp's instruction stream also missed the instruction cache more.  Packed: 25, 20 and 27,
 // 20 lanes; shade 354 -> 27 + 233 us and 238 -> 18 + 102 us on that still's bounces 0 and 1,
-// 8.06 -> 0.73 + 3.25 ms and 3.48 -> 0.22 + 0.37 ms on the batch's.
+// 8.06 -> 0.73 + 3.25 ms and 3.48 -> 0.22 + 0.37 ms on the batch's (one entry a thread).
 // The bounce's queue counters are reset here too: no kernel reads them between their last
 // reader and this one.
 constexpr int SPLIT_BLOCK = 512;
+constexpr uint32_t SPLIT_EACH = 2;   // entries per thread and pass, their loads in flight together
 constexpr int PATHS_BLOCKS = 2;   // blocks of k_paths per SM
 template <bool BATCH, bool EXT>
 __global__ void __launch_bounds__(SPLIT_BLOCK) k_split(const __grid_constant__ PathParams p, int cur) {
-    __shared__ uint32_t warp_hits[SPLIT_BLOCK / 32], base;
+    constexpr uint32_t WARPS = SPLIT_BLOCK / 32, NONE = 0xffffffffu;
+    static_assert(WARPS * SPLIT_EACH == 32u, "one warp scans the counts");
+    __shared__ uint32_t warp_hits[32], base;
     if (blockIdx.x == 0 && threadIdx.x == 0) { p.counters[cur ^ 1] = 0u; p.counters[2] = 0u; p.counters[11] = 0u; p.counters[12] = 0u; }
     const uint32_t n = p.counters[14] ? 0u : p.counters[cur], lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     uint32_t* hits = reinterpret_cast<uint32_t*>(p.ray_o[cur]);
-    for (uint32_t first = blockIdx.x * SPLIT_BLOCK; first < n; first += gridDim.x * SPLIT_BLOCK) {
-        const uint32_t i = first + threadIdx.x;
-        const uint32_t inst = i < n ? p.hit_inst[i] : 0xffffffffu;
-        const bool hit = inst != 0xffffffffu;
-        const uint32_t mask = __ballot_sync(0xffffffffu, hit);
-        if (lane == 0u) warp_hits[warp] = uint32_t(__popc(mask));
+    for (uint32_t first = blockIdx.x * (SPLIT_BLOCK * SPLIT_EACH); first < n; first += gridDim.x * (SPLIT_BLOCK * SPLIT_EACH)) {
+        uint32_t inst[SPLIT_EACH], slot[SPLIT_EACH], mask[SPLIT_EACH];
+        float4 rd[SPLIT_EACH], T[SPLIT_EACH], R[SPLIT_EACH];
+        #pragma unroll
+        for (uint32_t u = 0; u < SPLIT_EACH; ++u) {
+            const uint32_t i = first + u * SPLIT_BLOCK + threadIdx.x;
+            inst[u] = i < n ? p.hit_inst[i] : NONE;
+            rd[u] = p.ray_d[cur][min(i, n - 1u)];
+        }
+        #pragma unroll
+        for (uint32_t u = 0; u < SPLIT_EACH; ++u) {
+            slot[u] = __float_as_uint(rd[u].w);
+            T[u] = p.thr[slot[u]];
+            R[u] = p.rad[slot[u]];
+            mask[u] = __ballot_sync(0xffffffffu, inst[u] != NONE);
+            if (lane == 0u) warp_hits[u * WARPS + warp] = uint32_t(__popc(mask[u]));
+        }
         __syncthreads();
         if (warp == 0u) {
-            const uint32_t own = lane < SPLIT_BLOCK / 32 ? warp_hits[lane] : 0u;
+            const uint32_t own = warp_hits[lane];
             uint32_t sum = own;
             for (int off = 1; off < 32; off <<= 1) {
                 const uint32_t v = __shfl_up_sync(0xffffffffu, sum, off);
                 if (lane >= uint32_t(off)) sum += v;
             }
-            if (lane < SPLIT_BLOCK / 32) warp_hits[lane] = sum - own;
+            warp_hits[lane] = sum - own;
             if (lane == 31u) base = sum ? atomicAdd(&p.counters[13], sum) : 0u;
         }
         __syncthreads();
-        if (hit) hits[base + warp_hits[warp] + uint32_t(__popc(mask & ((1u << lane) - 1u)))] = i;
+        #pragma unroll
+        for (uint32_t u = 0; u < SPLIT_EACH; ++u)
+            if (inst[u] != NONE)
+                hits[base + warp_hits[u * WARPS + warp] + uint32_t(__popc(mask[u] & ((1u << lane) - 1u)))] = first + u * SPLIT_BLOCK + threadIdx.x;
         __syncthreads();   // the next pass writes warp_hits and base
-        if (i >= n) continue;
-        const bool ids = !BATCH ? p.job0.primary_ids != nullptr : true;
-        if (hit && !ids) continue;
-        const float4 rd = p.ray_d[cur][i];
-        const uint32_t slot = __float_as_uint(rd.w);
-        const Job& J = BATCH ? p.jobs[job_of_slot<true>(p, slot)] : p.job0;
-        const float4 T = p.thr[slot];
-        const uint32_t bounce = __float_as_uint(T.w) & 0xffu;
-        if (J.primary_ids && bounce == 0u) store_ids(J, slot, inst, hit ? __float_as_uint(p.hit[i].w) : 0u);
-        if (hit) continue;
-        finish_miss<EXT>(p, J, slot, f3(rd.x, rd.y, rd.z), T, bounce);
+        #pragma unroll
+        for (uint32_t u = 0; u < SPLIT_EACH; ++u) {
+            const uint32_t i = first + u * SPLIT_BLOCK + threadIdx.x;
+            if (i >= n) break;
+            const bool hit = inst[u] != NONE;
+            const Job& J = BATCH ? p.jobs[job_of_slot<true>(p, slot[u])] : p.job0;
+            const uint32_t bounce = __float_as_uint(T[u].w) & 0xffu;
+            if (bounce == 0u && J.primary_ids) store_ids(J, slot[u], inst[u], hit ? __float_as_uint(p.hit[i].w) : 0u);
+            if (!hit) finish_miss<EXT>(p, J, slot[u], f3(rd[u].x, rd[u].y, rd[u].z), T[u], R[u], bounce);
+        }
     }
 }
 
@@ -1597,7 +1614,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, PATHS_BLOCKS) k_paths(const __gri
             if (J.primary_ids && b == 0u) store_ids(J, slot, inst, __float_as_uint(hh.w));
             if (inst == 0xffffffffu) {
                 const float4 T = p.thr[slot];
-                finish_miss<EXT>(p, J, slot, out.d, T, __float_as_uint(T.w) & 0xffu);
+                finish_miss<EXT>(p, J, slot, out.d, T, p.rad[slot], __float_as_uint(T.w) & 0xffu);
             } else {
                 shade_vertex<EXT>(p, J, slot, out.d, hh, inst, out);
             }
