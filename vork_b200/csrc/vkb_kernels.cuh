@@ -637,6 +637,7 @@ __device__ __forceinline__ uint32_t find_job(const PathParams& p, uint32_t x) {
 // 33.8 ms); tiles of 4 or 8 image rows under this order: equal or 1% slower.
 template <bool BATCH>
 __global__ void k_camera(PathParams p) {
+    cudaGridDependencySynchronize();
     const uint32_t n = p.counters[7];
     for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < n; slot += gridDim.x * blockDim.x) {
         uint32_t j = BATCH ? find_job<false>(p, slot) : 0u;
@@ -749,6 +750,7 @@ __device__ __forceinline__ uint32_t share_index(uint32_t share) {
 // the same way, 256x256 16 spp 2.72 -> 2.37 ms.
 template <bool COUNT, bool BATCH, bool W8 = false>
 __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace(PathParams p, int cur) {
+    cudaGridDependencySynchronize();
     VKB_STACK_DECL_W(W8)
     const uint32_t n = p.counters[14] ? 0u : p.counters[cur];
     if (blockIdx.x == 0 && threadIdx.x == 0) { atomicAdd(&p.counters[3], n); p.counters[13] = 0u; }
@@ -877,6 +879,7 @@ struct ShadowLane {
 // EXT: waves with an image environment or emissive meshes.
 template <bool COUNT, bool BATCH, bool EXT, bool W8 = false>
 __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace_shadow(PathParams p) {
+    cudaGridDependencySynchronize();
     VKB_STACK_DECL_W(W8)
     const uint32_t n = p.counters[2];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&p.counters[4], n);
@@ -1233,6 +1236,7 @@ constexpr uint32_t SPLIT_EACH = 2;   // entries per thread and pass, their loads
 constexpr int PATHS_BLOCKS = 2;   // blocks of k_paths per SM
 template <bool BATCH, bool EXT>
 __global__ void __launch_bounds__(SPLIT_BLOCK) k_split(const __grid_constant__ PathParams p, int cur) {
+    cudaGridDependencySynchronize();
     constexpr uint32_t WARPS = SPLIT_BLOCK / 32, NONE = 0xffffffffu;
     static_assert(WARPS * SPLIT_EACH == 32u, "one warp scans the counts");
     __shared__ uint32_t warp_hits[32], base;
@@ -1547,6 +1551,7 @@ constexpr int SHADE_BLOCK = VKB_SHADE_BLOCK;
 // resident: the blocks that run at once; a short hit list is spread over their warps.
 template <bool BATCH, bool EXT>
 __global__ void __launch_bounds__(VKB_SHADE_BLOCK, VKB_SHADE_MIN_BLOCKS) k_shade(const __grid_constant__ PathParams p, int cur, uint32_t resident) {
+    cudaGridDependencySynchronize();
     QueueOut out{p, cur ^ 1};
     const uint32_t n = p.counters[13];
     const uint32_t* hits = reinterpret_cast<const uint32_t*>(p.ray_o[cur]);
@@ -1583,6 +1588,7 @@ struct LaneOut {
 // it takes it, counters[14] tells this bounce's kernels that the queue is empty.
 template <bool EXT, bool W8>
 __global__ void __launch_bounds__(TRACE_BLOCK, PATHS_BLOCKS) k_paths(const __grid_constant__ PathParams p, uint32_t first, uint32_t bounces, uint32_t most) {
+    cudaGridDependencySynchronize();
     VKB_STACK_DECL_W(W8)
     const int cur = int(first & 1u);
     const uint32_t n = p.counters[cur], lane = threadIdx.x & 31u;
@@ -1642,6 +1648,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, PATHS_BLOCKS) k_paths(const __gri
 }
 // Seed the first ray queue's count from the wave's path-slot count.
 __global__ void k_start_wave(uint32_t* counters, uint32_t append_camera) {
+    cudaGridDependencySynchronize();
     counters[0] = append_camera ? 0u : counters[7];
     counters[9] = 0u;
     counters[11] = 0u;   // trace fetch counters (closest, shadow)
@@ -1654,6 +1661,7 @@ __global__ void k_start_wave(uint32_t* counters, uint32_t append_camera) {
 // parity slot (i & 1) and stops once it and its whole 3x3 neighbourhood were settled at
 // the previous sample (slot (i & 1) ^ 1, which nothing writes during this kernel).
 __global__ void k_adaptive_decide(PathParams p) {
+    cudaGridDependencySynchronize();
     const Job& J = p.job0;
     const uint32_t i = J.wave_first, w = J.cam.width, h = J.cam.height;
     uint32_t skipped = 0;
@@ -1723,6 +1731,7 @@ __global__ void k_guides(PathParams p) {
 // one sample at a time in sample order (any wave size gives the same sums).
 template <bool BATCH>
 __global__ void k_accumulate(PathParams p) {
+    cudaGridDependencySynchronize();
     const uint32_t n = p.counters[8];
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < n; g += gridDim.x * blockDim.x) {
         const Job& J = BATCH ? p.jobs[find_job<true>(p, g)] : p.job0;
