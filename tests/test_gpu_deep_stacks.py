@@ -1,0 +1,42 @@
+"""Traversal stacks on trees as deep as they get: a geometric series of triangles, whose
+trees are chains.  Stack needs were counted on the CPU from the same trees."""
+import numpy as np
+import pytest
+
+from vork_b200 import abi, scene as S
+
+pytestmark = pytest.mark.gpu
+RATIO, FIRST = 1.25, 1e-3
+
+
+def _chain(renderer, count, **kw):
+    # Triangle i: (x, 0, 0), (x, 0, x), (x, x, 0) at x = FIRST * RATIO^i, so the ray from the
+    # origin along (1, a, a) crosses every triangle for a < 0.5 and every box for a < 1.
+    x = (FIRST * RATIO ** np.arange(count)).astype(np.float32)
+    z = np.zeros_like(x)
+    pos = np.stack([np.stack([x, z, z], 1), np.stack([x, z, x], 1), np.stack([x, x, z], 1)], 1).reshape(-1, 3)
+    nrm = np.tile(np.float32([-1, 0, 0]), (3 * count, 1))
+    sc = S.spheres_scene(num_spheres=1, width=16, height=16)
+    sc.meshes = [S.Mesh(pos, nrm, np.arange(3 * count, dtype=np.uint32).reshape(-1, 3))]
+    sc.instance_rows = S.rows_from(1.0, (0.0, 0.0, 0.0)).reshape(1, 3, 4)
+    sc.instance_mesh = sc.instance_material = np.zeros(1, np.uint32)
+    for k, v in kw.items():
+        setattr(sc, k, v)
+    return renderer.install(sc)
+
+
+def _ray(a):
+    d = np.array([1.0, a, a]) / np.sqrt(1 + 2 * a * a)
+    return np.concatenate([[0, 0, 0], d, [1e30]]).astype(np.float32)[None]
+
+
+@pytest.mark.parametrize("count,need", [(100, 85), (141, 120), (144, 122), (150, 127)])
+def test_8wide_stack_holds_128_entries(renderer, count, need):
+    # `need` entries are on the stack when the first leaf, the nearest triangle, is reached.
+    with _chain(renderer, count, blas_format=abi.BLAS_WIDE8) as s:
+        t, ids, _ = s.trace(_ray(0.3))
+        assert ids.tolist() == [[0, 0]]
+        assert abs(t[0] / (FIRST * np.sqrt(1.18)) - 1) < 1e-5
+        assert s.occluded(_ray(0.3)).all() and not s.occluded(_ray(0.6)).any()
+
+

@@ -58,19 +58,16 @@ struct MeshInfo {
 #ifndef VKB_SMEM_STACK
 #define VKB_SMEM_STACK 16
 #endif
-#ifndef VKB_SPILL_STACK
-#define VKB_SPILL_STACK 48
-#endif
 // Traversal stacks: the first SMEM_STACK entries live in shared memory as
 // [entry][thread] (lane l of a 128-thread block always touches bank l, whatever depth
-// each lane is at: no bank conflicts); deeper entries go to a per-thread local array of
-// SPILL_STACK entries.  Shared memory not taken by stacks serves as L1 for the nodes.
+// each lane is at: no bank conflicts); deeper entries go to a per-thread local array.
+// Shared memory not taken by stacks serves as L1 for the nodes.  The capacities do not
+// depend on that split: a tree that fits one split fits every other.  An 8-wide BLAS visit
+// pushes up to seven children: its traversals get twice the stack.
 constexpr int SMEM_STACK = VKB_SMEM_STACK;
-constexpr int SPILL_STACK = VKB_SPILL_STACK;
-constexpr int STACK_CAP = SMEM_STACK + SPILL_STACK;
-// An 8-wide BLAS visit pushes up to seven children: its traversals get a deeper local part.
-constexpr int SPILL_STACK8 = 104;
-constexpr int STACK_CAP8 = SMEM_STACK + SPILL_STACK8;
+constexpr int STACK_CAP = 64, STACK_CAP8 = 128;
+constexpr int SPILL_STACK = STACK_CAP - SMEM_STACK, SPILL_STACK8 = STACK_CAP8 - SMEM_STACK;
+static_assert(SPILL_STACK >= 0, "the shared part is within the stack");
 constexpr int TRACE_BLOCK = 128;
 // The ray in world space (origin, direction, their slab terms) is kept there the same way:
 // an instance entry reads the first two and its end the last two, instead of the queue entry
