@@ -40,3 +40,10 @@ def test_8wide_stack_holds_128_entries(renderer, count, need):
         assert s.occluded(_ray(0.3)).all() and not s.occluded(_ray(0.6)).any()
 
 
+@pytest.mark.parametrize("count", [100, 200, 220])
+def test_any_hit_rays_need_no_more_stack_than_sorted_children(renderer, count):
+    # A PLOC chain takes two triangles a level.  From the near end a ray that visits every
+    # child far to near has at most three entries waiting; one that takes the chain ahead of
+    # a nearer leaf has one more a level, and 64 hold.
+    with _chain(renderer, count, blas_builder=abi.BLAS_BUILD_PLOC) as s:
+        assert s.occluded(_ray(0.3)).all() and not s.occluded(_ray(0.6)).any()

@@ -178,6 +178,10 @@ __device__ __forceinline__ uint32_t slot_key(float nx, float ny, float nz, float
     float tf = min3f(fmaf(fx, r.idir.x, -r.ood.x), fmaf(fy, r.idir.y, -r.ood.y), fminf(fmaf(fz, r.idir.z, -r.ood.z), tmax));
     return tn <= tf * 1.00000024f ? ((__float_as_uint(tn) & ~3u) | k) : 0xffffffffu;
 }
+// Far-first key (larger entry distance, smaller key; misses stay ~0u).
+__device__ __forceinline__ uint32_t far_key(uint32_t key) {
+    return key == 0xffffffffu ? key : ((0x7ffffffcu - (key & ~3u)) | (key & 3u));
+}
 __device__ __forceinline__ void key_order(uint32_t& a, uint32_t& b) { uint32_t l = min(a, b); b = max(a, b); a = l; }
 __device__ __forceinline__ int slot_child(const int4& c, uint32_t key) {
     const bool odd = (key & 1u) != 0u;
@@ -267,7 +271,9 @@ struct TraceLane {
     RaySpace rs;
     float tbest;
     int node = DONE, sp;
-    bool found, in_blas, cull;
+    bool found, in_blas;
+    bool cull;      // closest hits: the instance's back faces do not count
+    bool ordered;   // occlusion rays: every child in order (see fail)
     const Bvh4Node* nodes;
     const Bvh8Node* nodes8;
     uint32_t tri_base, cur_instance, steps;
@@ -278,7 +284,7 @@ struct TraceLane {
         make_space(rs, o, d, false);
         stk.keep(WORLD_ORIGIN, o); stk.keep(WORLD_DIR, d); stk.keep(WORLD_IDIR, rs.idir); stk.keep(WORLD_OOD, rs.ood);
         tbest = tmax; sp = 0; steps = 0;
-        found = false; in_blas = false; cull = false;
+        found = false; in_blas = false; cull = false; ordered = false;
         nodes = s.tlas_nodes; tri_base = 0; cur_instance = 0;
         const bool any = s.num_instances != 0;
         node = any ? 0 : DONE;
@@ -286,7 +292,20 @@ struct TraceLane {
     }
     __device__ __forceinline__ bool done() const { return node == DONE; }
     __device__ __forceinline__ bool at_special() const { return node < 0 && node != DONE; }
-    __device__ __forceinline__ void fail(uint32_t* err, uint32_t bit) { atomicOr(err, bit); node = DONE; }
+    // Out of stack or steps.  An occlusion ray that took its children in the cheap order
+    // (visit) starts again with all of them far to near: how many entries wait, and what is
+    // met before a hit, depends on the order, and a chain-like tree that fits the stack in
+    // this one need not fit it in that one.
+    __device__ __forceinline__ void fail(uint32_t* err, uint32_t bit, TraceStack stk) {
+        if (ANY && !ordered) {
+            ordered = true; steps = 0;
+            stk.put(0, 0);   // the root, after an instance's end
+            sp = 1; node = LEAVE;
+            return;
+        }
+        atomicOr(err, bit);
+        node = DONE;
+    }
     __device__ __forceinline__ void pop(TraceStack stk) {
         if (sp == 0) { node = DONE; return; }
         --sp;
@@ -295,7 +314,7 @@ struct TraceLane {
     // A node (node >= 0): its nearest hit child next, the other hits pushed far to near, or
     // a pop when it has none.
     __device__ __forceinline__ void visit(uint32_t* err, TraceCount* count, TraceStack stk) {
-        if (++steps >= TRACE_STEP_LIMIT) { fail(err, 2u); return; }
+        if (++steps >= TRACE_STEP_LIMIT) { fail(err, 2u, stk); return; }
         if (W8 && in_blas) {
             // A compressed 8-wide BLAS node: decode the eight slots' planes on the ray's
             // grid (t = q * 2^e / d + (origin - o) / d), sort the hit slots' keys, descend
@@ -339,7 +358,7 @@ struct TraceLane {
                 int pushes = 0;
                 #pragma unroll
                 for (int i = 1; i < 8; ++i) pushes += key[i] != 0xffffffffu ? 1 : 0;
-                if (sp + pushes > CAP) { fail(err, 1u); return; }
+                if (sp + pushes > CAP) { fail(err, 1u, stk); return; }
                 #pragma unroll
                 for (int i = 7; i >= 1; --i)
                     if (key[i] != 0xffffffffu) { stk.put(sp, child(key[i])); ++sp; }
@@ -367,8 +386,19 @@ struct TraceLane {
                 // slot order: what they find does not depend on the order, so a sort is only
                 // worth its first place (a second of four hits is rare; with all four sorted
                 // 5.12 vs 5.00 ms for a 641x359 std/path still, 356.3 vs 355.1 ms for the flock
-                // frame).  A miss, ~0u, is the smallest as a signed key.
+                // frame).  A miss, ~0u, is the smallest as a signed key.  Both orders end at
+                // the same answer where both fit; a ray that runs out here takes the other.
                 const uint32_t far = uint32_t(max(max(int(k0), int(k1)), max(int(k2), int(k3))));
+                if (far != 0xffffffffu && ordered) {
+                    k0 = far_key(k0); k1 = far_key(k1); k2 = far_key(k2); k3 = far_key(k3);
+                    key_order(k0, k1); key_order(k2, k3); key_order(k0, k2); key_order(k1, k3); key_order(k1, k2);
+                    if (sp + int(k1 != 0xffffffffu) + int(k2 != 0xffffffffu) + int(k3 != 0xffffffffu) > CAP) { fail(err, 1u, stk); return; }
+                    if (k3 != 0xffffffffu) { stk.put(sp, slot_child(ch, k3)); ++sp; }
+                    if (k2 != 0xffffffffu) { stk.put(sp, slot_child(ch, k2)); ++sp; }
+                    if (k1 != 0xffffffffu) { stk.put(sp, slot_child(ch, k1)); ++sp; }
+                    node = slot_child(ch, k0);
+                    return;
+                }
                 if (far != 0xffffffffu) {
                     const bool p0 = k0 != 0xffffffffu && k0 != far, p1 = k1 != 0xffffffffu && k1 != far;
                     const bool p2 = k2 != 0xffffffffu && k2 != far, p3 = k3 != 0xffffffffu && k3 != far;
@@ -380,7 +410,7 @@ struct TraceLane {
                         if (p1) { *top = ch.y; top += TRACE_BLOCK; ++sp; }
                         if (p0) { *top = ch.x; ++sp; }
                     } else {
-                        if (sp + int(p0) + int(p1) + int(p2) + int(p3) > CAP) { fail(err, 1u); return; }
+                        if (sp + int(p0) + int(p1) + int(p2) + int(p3) > CAP) { fail(err, 1u, stk); return; }
                         if (p3) { stk.put(sp, ch.w); ++sp; }
                         if (p2) { stk.put(sp, ch.z); ++sp; }
                         if (p1) { stk.put(sp, ch.y); ++sp; }
@@ -403,7 +433,7 @@ struct TraceLane {
                         if (k2 != 0xffffffffu) { stk.r[sp * TRACE_BLOCK] = slot_child(ch, k2); ++sp; }
                         stk.r[sp * TRACE_BLOCK] = slot_child(ch, k1); ++sp;
                     } else {
-                        if (sp + pushes > CAP) { fail(err, 1u); return; }
+                        if (sp + pushes > CAP) { fail(err, 1u, stk); return; }
                         if (k3 != 0xffffffffu) { stk.put(sp, slot_child(ch, k3)); ++sp; }
                         if (k2 != 0xffffffffu) { stk.put(sp, slot_child(ch, k2)); ++sp; }
                         stk.put(sp, slot_child(ch, k1)); ++sp;
@@ -420,7 +450,7 @@ struct TraceLane {
     // for another one sets up the ray's space once.
     __device__ __forceinline__ void special(const SceneView& s, uint32_t* err, TraceCount* count, TraceStack stk) {
         if (in_blas && node != LEAVE) {
-            if (++steps >= TRACE_STEP_LIMIT) { fail(err, 2u); return; }
+            if (++steps >= TRACE_STEP_LIMIT) { fail(err, 2u, stk); return; }
             // BLAS leaf: up to VKB_BLAS_LEAF_MAX triangles in leaf order, ~((first << 2) | (count - 1)).
             uint32_t v = uint32_t(~node), first = v >> 2, cnt = VKB_BLAS_LEAF_MAX == 1 ? 1u : (v & 3u) + 1u;
             for (uint32_t k = 0; k < cnt; ++k) {
@@ -450,7 +480,7 @@ struct TraceLane {
             return;
         }
         // Instance entry: the ray in object space.
-        if (++steps >= TRACE_STEP_LIMIT) { fail(err, 2u); return; }
+        if (++steps >= TRACE_STEP_LIMIT) { fail(err, 2u, stk); return; }
         if (COUNT) count->instances++;
         const TlasLeaf* lf = s.tlas_leaves + (~node);
         float4 r0, r1, r2, in;
@@ -465,7 +495,7 @@ struct TraceLane {
         else nodes = s.blas_nodes + info.y;
         tri_base = info.z;
         cull = !ANY && (info.w & LEAF_CULL_BACKFACES);
-        if (sp >= CAP) { fail(err, 1u); return; }
+        if (sp >= CAP) { fail(err, 1u, stk); return; }
         stk.put(sp, LEAVE);
         ++sp;
         in_blas = true;
