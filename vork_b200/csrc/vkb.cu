@@ -29,6 +29,7 @@
 #include "vkb_kernels.cuh"
 #include "vkb_sah.h"
 #include "vkb_wide8.h"
+#include "vkb_graphs.h"
 #include "vkb_nrc.cuh"
 #include "vkb_display.cuh"
 
@@ -420,7 +421,6 @@ struct Wavefront {
         hit_inst.release(); slot_job.release(); rng.release(); counters.release(); err.release(); work.release(); jobs.release();
     }
 };
-struct GraphEntry { uint64_t key; cudaGraphExec_t exec; };
 
 constexpr size_t SINGLE_JOB_WAVE_SLOTS = size_t(64) << 20;   // 14.8 GB of queues per wavefront when full
 struct vkb_ctx {
@@ -1027,7 +1027,7 @@ struct WaveEngine {
     std::vector<Job> table;
     std::vector<Job> wave_table;        // the jobs of the current wave (uploaded)
     WaveTotals tot;
-    std::vector<GraphEntry> captured;   // this engine's wave graphs (they point at its buffers)
+    vkb_host::WaveGraphs<cudaGraphExec_t> graphs_kept;   // this engine's wave graphs (they point at its buffers)
     // Scheduling: fair (one sample of every unfinished job per wave, then more), packed
     // (each job's remaining samples before the next job: fewer scenes per wave, so their
     // BVHs stay in L2 -- batch throughput), or shortest remaining work first (the jobs
@@ -1035,7 +1035,7 @@ struct WaveEngine {
     bool packed = false, srpt = false;
     double aging_rate = 0.0;              // shortest-first aging, paths per second waited
     const CacheLaunch* cache = nullptr;   // radiance-cache hooks (single-job renders)
-    ~WaveEngine() { for (auto& g : captured) cudaGraphExecDestroy(g.exec); }
+    ~WaveEngine() { for (auto& g : graphs_kept.kept) cudaGraphExecDestroy(g.second); }
     WaveEngine(vkb_ctx* ctx, const WaveBuffers& wb, size_t cap, uint32_t fl, bool use_graphs) : c(ctx), w(wb), capacity(cap), flags(fl), graphs(use_graphs) {
         cudaStream_t st = c->stream;
         VKB_CUDA(cudaMemsetAsync(w.counters, 0, 16 * sizeof(uint32_t), st));
@@ -1178,24 +1178,24 @@ struct WaveEngine {
             p.cache = cache->dev;
         }
         if (use_graph) {
-            uint64_t key = (uint64_t(bounces) << 1) | 1u;
-            key = key * 1315423911ull + (counted ? 7u : 3u) + (ext ? 11u : 0u) + (w8 ? 17u : 0u);
-            key = key * 40503ull + wave_jobs;
             const WaveGrids grids(c, n_paths);
-            key = (key * 97ull + uint64_t(grids.trace)) * 19457ull + uint64_t(grids.shade);
-            cudaGraphExec_t exec = nullptr;
-            for (auto& g : captured) if (g.key == key) exec = g.exec;
+            vkb_host::WaveKey key;
+            key.bounces = bounces; key.jobs = wave_jobs;
+            key.counted = counted; key.ext = ext; key.w8 = w8;
+            key.trace = grids.trace; key.split = grids.split; key.shade = grids.shade;
+            cudaGraphExec_t* exec = graphs_kept.find(key);
             if (!exec) {
                 cudaGraph_t g;
+                cudaGraphExec_t made = nullptr;
                 VKB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
                 WaveTotals scratch;
                 wave_kernels<true>(c, p, n_paths, bounces, counted, false, scratch, nullptr, ext, w8);
                 VKB_CUDA(cudaStreamEndCapture(st, &g));
-                VKB_CUDA(cudaGraphInstantiate(&exec, g, 0));
+                VKB_CUDA(cudaGraphInstantiate(&made, g, 0));
                 VKB_CUDA(cudaGraphDestroy(g));
-                captured.push_back({key, exec});
+                exec = graphs_kept.add(key, made);
             }
-            VKB_CUDA(cudaGraphLaunch(exec, st));
+            VKB_CUDA(cudaGraphLaunch(*exec, st));
             tot.launches += 3 + 4 * (bounces + 1);
             tot.trace_launches += bounces + 1;
         } else if (batch) {
