@@ -31,3 +31,10 @@ def _serve(renderer, groups, spp=1):
 def test_a_wave_is_not_replayed_from_a_graph_of_another_job_count(renderer):
     # 2 x 7500 paths, then 3 x 4484: trace grids of 938 and 841 blocks, equal shade grids.
     _serve(renderer, [[(75, 100)] * 2, [(59, 76)] * 3, [(75, 100)] * 2])
+
+
+def test_waves_of_many_sizes_share_few_graphs(renderer):
+    # More waves than are kept, their sizes on both sides of the grids' powers of two.
+    rng = np.random.default_rng(5)
+    sizes = [(int(w), int(h)) for w, h in zip(rng.integers(20, 60, 24), rng.integers(20, 90, 24))] + [(32, 32), (33, 31), (64, 64), (65, 63)]
+    _serve(renderer, [[sizes[int(k)] for k in rng.integers(0, len(sizes), rng.integers(2, 9))] for _ in range(90)])

@@ -1,4 +1,4 @@
-"""The keys of the captured wave graphs (vork_b200/csrc/vkb_graphs.h), no GPU."""
+"""The captured wave graphs (vork_b200/csrc/vkb_graphs.h): keys and bounds, no GPU."""
 import shutil
 import subprocess
 from pathlib import Path
@@ -8,7 +8,7 @@ import pytest
 ROOT = Path(__file__).resolve().parent.parent
 
 
-def test_wave_graph_keys(tmp_path):
+def test_wave_graph_keys_and_bounds(tmp_path):
     gxx = shutil.which("g++")
     if not gxx:
         pytest.skip("needs g++")

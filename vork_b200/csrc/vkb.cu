@@ -1178,7 +1178,8 @@ struct WaveEngine {
             p.cache = cache->dev;
         }
         if (use_graph) {
-            const WaveGrids grids(c, n_paths);
+            const uint32_t slots = vkb_host::graph_slots(n_paths);
+            const WaveGrids grids(c, slots);
             vkb_host::WaveKey key;
             key.bounces = bounces; key.jobs = wave_jobs;
             key.counted = counted; key.ext = ext; key.w8 = w8;
@@ -1189,11 +1190,11 @@ struct WaveEngine {
                 cudaGraphExec_t made = nullptr;
                 VKB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
                 WaveTotals scratch;
-                wave_kernels<true>(c, p, n_paths, bounces, counted, false, scratch, nullptr, ext, w8);
+                wave_kernels<true>(c, p, slots, bounces, counted, false, scratch, nullptr, ext, w8);
                 VKB_CUDA(cudaStreamEndCapture(st, &g));
                 VKB_CUDA(cudaGraphInstantiate(&made, g, 0));
                 VKB_CUDA(cudaGraphDestroy(g));
-                exec = graphs_kept.add(key, made);
+                exec = graphs_kept.add(key, made, [](cudaGraphExec_t old) { cudaGraphExecDestroy(old); });
             }
             VKB_CUDA(cudaGraphLaunch(*exec, st));
             tot.launches += 3 + 4 * (bounces + 1);
