@@ -1,0 +1,70 @@
+// Test harness (tests only) of the kept device buffers, over an allocator of 1 GiB.
+#include <cstdio>
+#include <cstdlib>
+#include <map>
+#include <stdexcept>
+#include "vkb_pool.h"
+
+struct Api {
+    static size_t limit, used, calls;
+    static std::map<void*, size_t> live;
+    static void* alloc(size_t bytes) {
+        ++calls;
+        if (used + bytes > limit) return nullptr;
+        void* p = std::malloc(1);
+        live[p] = bytes;
+        used += bytes;
+        return p;
+    }
+    [[noreturn]] static void out_of_memory() { throw std::runtime_error("out of memory"); }
+    static void free(void* p) {
+        auto it = live.find(p);
+        if (it == live.end()) { std::printf("FAIL freed twice\n"); std::exit(1); }
+        used -= it->second;
+        live.erase(it);
+        std::free(p);
+    }
+};
+size_t Api::limit = size_t(1) << 30, Api::used = 0, Api::calls = 0;
+std::map<void*, size_t> Api::live;
+using Pool = vkb_host::DevicePool<Api>;
+constexpr size_t MIB = size_t(1) << 20;
+
+static int bad = 0;
+static void check(bool ok, const char* what) {
+    if (!ok) { std::printf("FAIL %s\n", what); ++bad; }
+}
+// As an object's buffers: from the pool if it has one, given back to it or freed.
+struct Buf { void* p; size_t bytes; };
+static Buf take(Pool& pool, size_t bytes) {
+    size_t b = bytes;
+    void* p = pool.take(b);
+    if (!p) p = vkb_host::device_alloc<Api>(b = bytes);
+    return {p, b};
+}
+static void drop(Pool& pool, Buf b) {
+    if (!pool.give(b.p, b.bytes)) Api::free(b.p);
+}
+
+static void allocations_trim() {
+    // 200 MiB idle in each of two pools, 600 MiB in use: 300 MiB more fit once both are emptied.
+    Pool a, b;
+    drop(a, take(a, 200 * MIB));
+    drop(b, take(b, 200 * MIB));
+    check(Api::used == 400 * MIB, "idle buffers are kept");
+    void* big = vkb_host::device_alloc<Api>(600 * MIB);
+    void* p = vkb_host::device_alloc<Api>(300 * MIB);
+    check(Api::used == 900 * MIB, "an allocation frees what is idle");
+    bool failed = false;
+    try { vkb_host::device_alloc<Api>(200 * MIB); } catch (const std::runtime_error&) { failed = true; }
+    check(failed && Api::used == 900 * MIB, "and then says that memory is out");
+    Api::free(big);
+    Api::free(p);
+}
+
+int main() {
+    allocations_trim();
+    check(Api::used == 0 && Api::live.empty(), "everything is given back");
+    if (!bad) std::printf("OK\n");
+    return bad;
+}

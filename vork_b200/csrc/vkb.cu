@@ -30,6 +30,7 @@
 #include "vkb_sah.h"
 #include "vkb_wide8.h"
 #include "vkb_graphs.h"
+#include "vkb_pool.h"
 #include "vkb_nrc.cuh"
 #include "vkb_display.cuh"
 
@@ -54,57 +55,20 @@ struct Unsupported { std::string msg; };
 struct InternalError { std::string msg; };
 struct DeviceTimeout { std::string msg; };
 
-// Device buffers that scenes and calls of one context gave back, for the next ones: an
-// install takes some forty buffers and a display call three, and cudaMalloc / cudaFree (which
-// waits for the device) took most of a small scene's install (20,000 birds on the GPU
-// builders, first frame of 640x360: 14-25 ms from process to process, 4.3 ms with kept
-// buffers).  Bounded; a buffer comes back only when no work on any stream still uses it; what
-// is idle is freed when the context closes or when any allocation runs out of memory.
-class DevicePool {
-public:
-    static constexpr size_t KEEP = size_t(256) << 20;   // idle bytes at most
-    DevicePool() { std::lock_guard<std::mutex> g(all_mutex()); all().push_back(this); }
-    ~DevicePool() {
-        { std::lock_guard<std::mutex> g(all_mutex()); all().erase(std::remove(all().begin(), all().end(), this), all().end()); }
-        trim();
+struct DeviceApi {
+    static void* alloc(size_t bytes) {
+        void* p = nullptr;
+        const cudaError_t e = cudaMalloc(&p, bytes);
+        if (e == cudaSuccess) return p;
+        cudaGetLastError();
+        if (e != cudaErrorMemoryAllocation) throw CudaError{e, "cudaMalloc"};
+        return nullptr;
     }
-    // An idle buffer of at least `bytes` (not twice that and more), or null; bytes: its size.
-    void* take(size_t& bytes) {
-        std::lock_guard<std::mutex> g(m_);
-        auto it = idle_.lower_bound(bytes);
-        if (it == idle_.end() || it->first > 2 * bytes + (size_t(64) << 10)) return nullptr;
-        void* p = it->second;
-        bytes = it->first;
-        held_ -= bytes;
-        idle_.erase(it);
-        return p;
-    }
-    // False when it would hold too much: the caller frees it.
-    bool give(void* p, size_t bytes) {
-        std::lock_guard<std::mutex> g(m_);
-        if (held_ + bytes > KEEP) return false;
-        idle_.emplace(bytes, p);
-        held_ += bytes;
-        return true;
-    }
-    void trim() {
-        std::lock_guard<std::mutex> g(m_);
-        for (auto& b : idle_) cudaFree(b.second);
-        idle_.clear();
-        held_ = 0;
-    }
-    static void trim_all() {
-        std::lock_guard<std::mutex> g(all_mutex());
-        for (DevicePool* p : all()) p->trim();
-    }
-
-private:
-    static std::mutex& all_mutex() { static std::mutex m; return m; }
-    static std::vector<DevicePool*>& all() { static std::vector<DevicePool*> v; return v; }
-    std::mutex m_;
-    std::multimap<size_t, void*> idle_;
-    size_t held_ = 0;
+    [[noreturn]] static void out_of_memory() { throw CudaError{cudaErrorMemoryAllocation, "cudaMalloc"}; }
+    static void free(void* p) { cudaFree(p); }
 };
+using DevicePool = vkb_host::DevicePool<DeviceApi>;
+void* device_alloc(size_t bytes) { return vkb_host::device_alloc<DeviceApi>(bytes); }
 
 template <class T> struct DBuf {
     T* p = nullptr;
@@ -119,15 +83,7 @@ template <class T> struct DBuf {
         if (count == 0) return;
         bytes = count * sizeof(T);
         void* q = pool ? pool->take(bytes) : nullptr;
-        if (!q) {
-            cudaError_t e = cudaMalloc(&q, bytes);
-            if (e == cudaErrorMemoryAllocation) {
-                cudaGetLastError();
-                DevicePool::trim_all();
-                e = cudaMalloc(&q, bytes);
-            }
-            if (e != cudaSuccess) throw CudaError{e, "cudaMalloc(&q, bytes)"};
-        }
+        if (!q) q = device_alloc(bytes);
         p = static_cast<T*>(q);
         n = count;
     }
@@ -2313,9 +2269,13 @@ vkb_server::Buffers take_buffers(vkb_server* v, size_t npix) {
     }
     vkb_server::Buffers b;
     b.npix = npix;
-    VKB_CUDA(cudaMalloc(&b.accum, npix * sizeof(float4)));
-    cudaError_t e = cudaMalloc(&b.out, npix * sizeof(float4));
-    if (e != cudaSuccess) { cudaFree(b.accum); throw CudaError{e, "cudaMalloc(request image)"}; }
+    b.accum = static_cast<float4*>(device_alloc(npix * sizeof(float4)));
+    try {
+        b.out = static_cast<float4*>(device_alloc(npix * sizeof(float4)));
+    } catch (...) {
+        cudaFree(b.accum);
+        throw;
+    }
     return b;
 }
 void free_pool(vkb_server* v) {
@@ -2471,6 +2431,7 @@ vkb_status vkb_server_step(vkb_server* v, vkb_server_status* status) {
                     size_t f = 0, t = 0;
                     return cudaMemGetInfo(&f, &t) == cudaSuccess ? uint64_t(f) : ~uint64_t(0);
                 };
+                if (device_free() < extra + ext_bytes + SERVER_DEVICE_RESERVE) DevicePool::trim_all();
                 if (device_free() < extra + ext_bytes + SERVER_DEVICE_RESERVE && v->pool_bytes) {
                     finished += reap(v, true, false);
                     free_pool(v);
