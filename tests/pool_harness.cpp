@@ -62,8 +62,25 @@ static void allocations_trim() {
     Api::free(p);
 }
 
+static void reuse_is_close_in_size() {
+    Pool pool;
+    const size_t idle[] = {100, 70000, 300000, 3 * MIB, 40 * MIB};
+    for (size_t b : idle) drop(pool, {Api::alloc(b), b});
+    const struct { size_t ask, got; } asks[] = {{60, 100}, {60, 60}, {150000, 300000}, {33 * MIB, 33 * MIB}, {3 * MIB - 5, 3 * MIB}, {39 * MIB, 40 * MIB}, {2000, 2000}, {4464, 70000}};
+    std::vector<Buf> held;
+    size_t before = Api::used;
+    for (const auto& a : asks) {
+        held.push_back(take(pool, a.ask));
+        check(held.back().bytes == (a.ask == 60 && held.size() == 2 ? 60 : a.got), "a buffer of about the size");
+        check(Api::live.at(held.back().p) == held.back().bytes, "its size is the allocation's");
+    }
+    check(Api::used - before == 60 + 33 * MIB + 2000, "the others are new");
+    for (const Buf& b : held) drop(pool, b);
+}
+
 int main() {
     allocations_trim();
+    reuse_is_close_in_size();
     check(Api::used == 0 && Api::live.empty(), "everything is given back");
     if (!bad) std::printf("OK\n");
     return bad;

@@ -46,3 +46,29 @@ def test_a_request_gets_the_memory_that_closed_scenes_left_idle():
                 rid = srv.submit(s, prof)
                 srv.run_until_idle()
             assert np.array_equal(srv.images[rid], want)
+
+
+def test_kept_buffers_count_as_allocated_and_never_refuse_a_request():
+    make = lambda n: S.spheres_scene(num_spheres=n, width=160, height=120, grid_cells=40)
+    prof = Profile.reference_transport(3, 1)
+    with Renderer(0) as r, r.install(make(50)) as s:
+        asked = s.info()["scene_bytes"]
+        want = s.render(prof).image
+    with Renderer(0) as r:
+        r.install(make(90)).close()
+        with r.install(make(50)) as s:
+            held = s.info()["scene_bytes"]
+            assert asked < held <= asked + 40 * MIB
+            cap = 160 * 120
+            with Server(r, memory_budget_bytes=1 << 40, max_jobs=4, wave_capacity=cap) as srv:
+                wave = srv.step()["used_bytes"]
+            # Just the room that the scene asked for: one request at a time, each to its end.
+            with Server(r, memory_budget_bytes=wave + asked + cap * 32, max_jobs=4, wave_capacity=cap) as srv:
+                ids = [srv.submit(s, prof) for _ in range(3)]
+                st = srv.step()
+                assert st["running"] == 1 and st["queued"] == 2 and st["used_bytes"] == wave + held + cap * 32
+                for _ in range(100):
+                    st = srv.step()
+                    if st["queued"] + st["running"] == 0:
+                        break
+                assert all(np.array_equal(srv.images[i], want) for i in ids)

@@ -73,24 +73,25 @@ void* device_alloc(size_t bytes) { return vkb_host::device_alloc<DeviceApi>(byte
 template <class T> struct DBuf {
     T* p = nullptr;
     size_t n = 0;
-    size_t bytes = 0;             // of the allocation
+    size_t bytes = 0;             // of the allocation (a kept buffer may be larger than asked for)
     DevicePool* pool = nullptr;   // where release() gives it back (none: freed)
     // Growing frees the old buffer rather than giving it back: queued work may still read it.
     void alloc(size_t count) {
         if (count <= n && p) return;
         if (p) cudaFree(p);
-        p = nullptr; n = 0;
+        p = nullptr; n = 0; bytes = 0;
         if (count == 0) return;
-        bytes = count * sizeof(T);
-        void* q = pool ? pool->take(bytes) : nullptr;
-        if (!q) q = device_alloc(bytes);
+        size_t size = count * sizeof(T);
+        void* q = pool ? pool->take(size) : nullptr;
+        if (!q) q = device_alloc(size);
         p = static_cast<T*>(q);
         n = count;
+        bytes = size;
     }
     // No work on any stream may still use it.
     void release() {
         if (p && !(pool && pool->give(p, bytes))) cudaFree(p);
-        p = nullptr; n = 0;
+        p = nullptr; n = 0; bytes = 0;
     }
     void upload(const T* src, size_t count, cudaStream_t s) { alloc(count); if (count) VKB_CUDA(cudaMemcpyAsync(p, src, count * sizeof(T), cudaMemcpyHostToDevice, s)); }
 };
@@ -490,6 +491,19 @@ template <class F> vkb_status guarded(F&& f) {
     } catch (const std::bad_alloc&) {
         return fail(VKB_OUT_OF_MEMORY, "host allocation failed");
     }
+}
+
+// Device bytes of a scene: what it holds itself whether a fork or not (instances and TLAS),
+// and what a fork shares with its base.  Counted as allocated, or as asked for: a kept buffer
+// of another scene may be the larger one.
+constexpr auto allocated = [](const auto& b) { return uint64_t(b.bytes); };
+constexpr auto asked = [](const auto& b) { return uint64_t(b.n * sizeof(*b.p)); };
+template <class Count> uint64_t own_bytes(const vkb_scene* s, Count size) {
+    return size(s->tlas_nodes) + size(s->tlas4) + size(s->tlas_odd) + size(s->tlas_leaves) + size(s->o2w) + size(s->w2o) + size(s->inst_info) + size(s->em_tree);
+}
+template <class Count> uint64_t shared_bytes(const vkb_scene* s, Count size) {
+    return size(s->vpos) + size(s->vnrm) + size(s->indices) + size(s->blas4) + size(s->blas8) + size(s->blas_tris) + size(s->tri_nrm) + size(s->env_img) +
+           size(s->env_dist) + size(s->em_inst_source) + size(s->em_sources);
 }
 
 SceneView scene_view(const vkb_scene* s) {
@@ -1952,12 +1966,7 @@ vkb_status vkb_scene_info(vkb_scene* s, vkb_scene_info_t* out) {
     out->tlas_rebuilds = s->tlas_rebuilds;
     out->tlas_refits = s->tlas_refits;
     out->motion_bytes = s->motion_bytes;
-    size_t dev = 0;
-    dev += s->vpos.n * sizeof(float4) + s->vnrm.n * sizeof(float4) + s->indices.n * 4 + s->blas4.n * sizeof(Bvh4Node) + s->blas8.n * sizeof(Bvh8Node) +
-           (s->blas_tris.n + s->tri_nrm.n) * sizeof(float4);
-    dev += s->tlas_nodes.n * sizeof(BvhNode) + s->tlas4.n * sizeof(Bvh4Node) + s->tlas_odd.n + s->tlas_leaves.n * sizeof(TlasLeaf) + (s->o2w.n + s->w2o.n) * sizeof(float4);
-    dev += s->env_img.n * sizeof(float4) + s->env_dist.n * sizeof(float2) + s->em_inst_source.n * 4 + s->em_sources.n * sizeof(uint2) + s->em_tree.n * sizeof(float);
-    out->scene_bytes = dev;
+    out->scene_bytes = own_bytes(s, allocated) + shared_bytes(s, allocated);
     out->build_ms = s->build_ms;
     out->install_ms = s->install_ms; out->blas_host_ms = s->blas_host_ms; out->upload_ms = s->upload_ms; out->tlas_ms = s->tlas_ms;
     return VKB_OK;
@@ -2242,14 +2251,8 @@ struct vkb_server {
 
 namespace {
 // Device bytes a scene holds itself (a fork: its instances and TLAS only).
-uint64_t scene_bytes(const vkb_scene* s) {
-    uint64_t own = s->tlas_nodes.n * sizeof(BvhNode) + s->tlas4.n * sizeof(Bvh4Node) + s->tlas_odd.n + s->tlas_leaves.n * sizeof(TlasLeaf) +
-                   (s->o2w.n + s->w2o.n) * sizeof(float4) + s->inst_info.n * sizeof(uint4) + s->em_tree.n * sizeof(float);
-    if (s->base) return own;
-    return own + s->vpos.n * sizeof(float4) + s->vnrm.n * sizeof(float4) + s->indices.n * 4 + s->blas4.n * sizeof(Bvh4Node) + s->blas8.n * sizeof(Bvh8Node) +
-           (s->blas_tris.n + s->tri_nrm.n) * sizeof(float4) + s->env_img.n * sizeof(float4) + s->env_dist.n * sizeof(float2) +
-           s->em_inst_source.n * 4 + s->em_sources.n * sizeof(uint2);
-}
+template <class Count> uint64_t scene_bytes(const vkb_scene* s, Count size) { return own_bytes(s, size) + (s->base ? 0u : shared_bytes(s, size)); }
+uint64_t scene_bytes(const vkb_scene* s) { return scene_bytes(s, allocated); }
 uint64_t resident_bytes(const vkb_server* v) {
     uint64_t b = 0;
     for (auto& kv : v->resident) b += kv.second;
@@ -2375,7 +2378,7 @@ vkb_status vkb_server_submit_view(vkb_server* v, vkb_scene* s, const vkb_camera*
         if (s->blas8.p) throw Unsupported{"compressed 8-wide BLAS scenes render through vkb_render and vkb_render_batch"};
         const vkb_camera& c = cam ? *cam : s->camera;
         uint64_t need = uint64_t(c.width) * c.height * 32u;
-        const uint64_t sb = scene_bytes(s) + (s->base ? scene_bytes(s->base) : 0u);
+        const uint64_t sb = scene_bytes(s, asked) + (s->base ? scene_bytes(s->base, asked) : 0u);
         if (v->budget && v->wave_bytes + sb + need > v->budget) throw ArgError{"request can never fit the memory budget"};
         if (uint64_t(c.width) * c.height > v->capacity) throw ArgError{"request image larger than a wave"};
         *id = v->next_id++;
@@ -2407,8 +2410,12 @@ vkb_status vkb_server_step(vkb_server* v, vkb_server_status* status) {
             auto& q = v->queue.front();
             uint64_t npix = uint64_t(q.cam.width) * q.cam.height;
             uint64_t need = npix * SERVER_BYTES_PER_PIXEL;
-            uint64_t scene = v->resident.count(q.s) ? 0u : scene_bytes(q.s);
-            if (q.s->base && !v->resident.count(q.s->base)) scene += scene_bytes(q.s->base);
+            // A request that nothing runs beside is admitted by what its scene asked for, as it
+            // was at submission: kept buffers, which may be larger, never make it wait for good.
+            const bool alone = eng.jobs.empty() && v->inflight.empty();
+            auto bytes_of = [&](const vkb_scene* sc) { return alone ? scene_bytes(sc, asked) : scene_bytes(sc); };
+            uint64_t scene = v->resident.count(q.s) ? 0u : bytes_of(q.s);
+            if (q.s->base && !v->resident.count(q.s->base)) scene += bytes_of(q.s->base);
             auto held = [&] { return v->wave_bytes + resident_bytes(v) + v->used_bytes + v->pool_bytes; };
             auto fit = v->pool.lower_bound(npix);
             uint64_t extra = (fit != v->pool.end() && fit->first <= 2 * npix) ? 0u : need;   // reused buffers add nothing

@@ -26,11 +26,12 @@ public:
         { std::lock_guard<std::mutex> g(all_mutex()); all().erase(std::remove(all().begin(), all().end(), this), all().end()); }
         trim();
     }
-    // An idle buffer of at least `bytes` (not twice that and more), or null; bytes: its size.
+    // An idle buffer of at least `bytes`, or null; bytes: its size.  Not twice that and more,
+    // nor a MiB more: some forty buffers then hold at most 40 MiB that their scene did not ask for.
     void* take(size_t& bytes) {
         std::lock_guard<std::mutex> g(m_);
         auto it = idle_.lower_bound(bytes);
-        if (it == idle_.end() || it->first > 2 * bytes + (size_t(64) << 10)) return nullptr;
+        if (it == idle_.end() || it->first > bytes + std::min(bytes + (size_t(64) << 10), size_t(1) << 20)) return nullptr;
         void* p = it->second;
         bytes = it->first;
         held_ -= bytes;
