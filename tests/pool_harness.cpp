@@ -78,9 +78,29 @@ static void reuse_is_close_in_size() {
     for (const Buf& b : held) drop(pool, b);
 }
 
+static void small_scenes_after_a_large_one() {
+    // A scene of 300 MiB in buffers of 10 MiB leaves the pool full; scenes of forty small
+    // buffers, one after another, then still find theirs.
+    Pool pool;
+    std::vector<Buf> large;
+    for (int k = 0; k < 30; ++k) large.push_back(take(pool, 10 * MIB));
+    for (const Buf& b : large) drop(pool, b);
+    check(Api::used == 250 * MIB, "as many as the bound allows");
+    for (int turn = 0; turn < 4; ++turn) {
+        const size_t before = Api::calls;
+        std::vector<Buf> small;
+        for (size_t k = 1; k <= 40; ++k) small.push_back(take(pool, k * 100000));
+        check(turn == 0 || Api::calls == before, "a small scene's buffers are kept");
+        for (const Buf& b : small) drop(pool, b);
+        check(Api::used <= Pool::KEEP, "within the bound");
+    }
+    check(!pool.give(large[0].p, Pool::KEEP + 1), "a buffer above the bound is refused");
+}
+
 int main() {
     allocations_trim();
     reuse_is_close_in_size();
+    small_scenes_after_a_large_one();
     check(Api::used == 0 && Api::live.empty(), "everything is given back");
     if (!bad) std::printf("OK\n");
     return bad;

@@ -5,6 +5,7 @@
 #pragma once
 #include <algorithm>
 #include <cstddef>
+#include <cstdint>
 #include <map>
 #include <mutex>
 #include <vector>
@@ -32,23 +33,31 @@ public:
         std::lock_guard<std::mutex> g(m_);
         auto it = idle_.lower_bound(bytes);
         if (it == idle_.end() || it->first > bytes + std::min(bytes + (size_t(64) << 10), size_t(1) << 20)) return nullptr;
-        void* p = it->second;
+        void* p = it->second.p;
         bytes = it->first;
         held_ -= bytes;
         idle_.erase(it);
         return p;
     }
-    // False when it would hold too much: the caller frees it.
+    // Keeps the buffer, in place of those idle for longest where the bound asks for it (one
+    // large scene's buffers would otherwise keep every later scene's out for good).  False
+    // for a buffer above the bound itself: the caller frees it.
     bool give(void* p, size_t bytes) {
         std::lock_guard<std::mutex> g(m_);
-        if (held_ + bytes > KEEP) return false;
-        idle_.emplace(bytes, p);
+        if (bytes > KEEP) return false;
+        while (held_ + bytes > KEEP) {
+            auto oldest = std::min_element(idle_.begin(), idle_.end(), [](const auto& a, const auto& b) { return a.second.since < b.second.since; });
+            Api::free(oldest->second.p);
+            held_ -= oldest->first;
+            idle_.erase(oldest);
+        }
+        idle_.emplace(bytes, Idle{p, gives_++});
         held_ += bytes;
         return true;
     }
     void trim() {
         std::lock_guard<std::mutex> g(m_);
-        for (auto& b : idle_) Api::free(b.second);
+        for (auto& b : idle_) Api::free(b.second.p);
         idle_.clear();
         held_ = 0;
     }
@@ -61,8 +70,10 @@ private:
     static std::mutex& all_mutex() { static std::mutex m; return m; }
     static std::vector<DevicePool*>& all() { static std::vector<DevicePool*> v; return v; }
     std::mutex m_;
-    std::multimap<size_t, void*> idle_;
+    struct Idle { void* p; uint64_t since; };   // since: the give() it came with
+    std::multimap<size_t, Idle> idle_;
     size_t held_ = 0;
+    uint64_t gives_ = 0;
 };
 
 // New device memory.  Before it gives up, what every context's pool holds idle goes back.
