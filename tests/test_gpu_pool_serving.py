@@ -4,7 +4,7 @@ import contextlib
 import numpy as np
 import pytest
 
-from vork_b200 import Profile, Renderer, scene as S
+from vork_b200 import Profile, Renderer, abi, scene as S
 from vork_b200.serving import Server
 
 pytestmark = pytest.mark.gpu
@@ -72,3 +72,24 @@ def test_kept_buffers_count_as_allocated_and_never_refuse_a_request():
                     if st["queued"] + st["running"] == 0:
                         break
                 assert all(np.array_equal(srv.images[i], want) for i in ids)
+
+
+def test_a_fork_that_runs_out_of_memory_leaves_its_base(renderer):
+    # 2^26 emissive triangles: each fork needs a weight tree of 512 MiB of its own.
+    sc = S.spheres_scene(num_spheres=1, width=48, height=32)
+    sc.meshes = [S.grid((1.0, 1.0), (256, 128))]
+    sc.instance_rows = np.stack([S.rows_from(1.0, (i % 32 - 16.0, 0.0, i // 32 - 16.0)) for i in range(1024)])
+    sc.instance_mesh = sc.instance_material = np.zeros(1024, np.uint32)
+    sc.materials = [S.emissive(luminance=2.0, double_sided=True)]
+    sc.blas_builder = abi.BLAS_BUILD_LBVH
+    prof = Profile.reference_transport(2, 2)
+    with renderer.install(sc) as s:
+        assert sc.num_triangles == 1 << 26
+        want = s.render(prof).image
+        s.fork().close()
+        renderer.install(S.spheres_scene(num_spheres=2, width=16, height=16)).close()
+        with _device_memory_left(256 * MIB):
+            with pytest.raises(abi.VkbError) as e:
+                s.fork()
+            assert e.value.status == abi.VKB_OUT_OF_MEMORY
+        assert want[..., :3].max() > 0 and np.array_equal(s.render(prof).image, want)

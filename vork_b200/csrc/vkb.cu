@@ -1708,6 +1708,10 @@ vkb_status vkb_scene_fork(vkb_scene* b, vkb_scene** out) {
         s->mesh_info = b->mesh_info; s->inst_mesh = b->inst_mesh; s->inst_mat = b->inst_mat;
         s->materials = b->materials; s->lights = b->lights; s->camera = b->camera; s->env = b->env;
         s->tree_nodes = b->tree_nodes; s->tlas_builder = b->tlas_builder;
+        // From here on its destruction leaves the base's buffers alone, on the way out of a
+        // failed allocation too.
+        s->base = b;
+        b->forks++;
         // Shared, read-only: geometry, BLASes, materials, lights, light tree.
         s->vpos = b->vpos; s->vnrm = b->vnrm; s->blas_tris = b->blas_tris; s->tri_nrm = b->tri_nrm;
         s->indices = b->indices; s->meshes = b->meshes; s->blas4 = b->blas4; s->blas8 = b->blas8; s->blas_format = b->blas_format; s->blas_builder = b->blas_builder;
@@ -1717,8 +1721,6 @@ vkb_status vkb_scene_fork(vkb_scene* b, vkb_scene** out) {
         s->em_inst_source = b->em_inst_source; s->em_sources = b->em_sources;
         s->em_count = b->em_count; s->em_tris = b->em_tris; s->em_leaves = b->em_leaves;
         if (s->em_leaves) s->em_tree.alloc(2 * size_t(s->em_leaves));
-        s->base = b;
-        b->forks++;
         // Owned: the base's current instance rows and records, and a TLAS over them.
         uint32_t n = b->num_instances;
         s->inst_info.alloc(std::max(1u, n));
