@@ -240,7 +240,8 @@ typedef struct vkb_stats {
     float render_ms;           /* device time of the wavefront, CUDA events */
     float build_ms;            /* device time of the last acceleration-structure build */
     float trace_ms;            /* VKB_PROFILE_TIME_KERNELS: summed closest-hit trace kernel time */
-    uint32_t trace_launches;   /* closest-hit trace launches in this render */
+    uint32_t trace_launches;   /* closest-hit trace launches in this render (a small wave's bounces that run in
+                                  one launch have none of their own) */
     uint32_t kernel_launches;  /* every kernel this library launched for this render */
     uint64_t nodes_visited;    /* VKB_PROFILE_COUNT_TRAVERSAL: closest-hit BVH node visits */
     uint64_t triangles_tested; /* closest-hit triangle tests */
@@ -508,6 +509,9 @@ vkb_status vkb_debug_trace(vkb_scene* scene, uint32_t n, const float* rays7, flo
  * ACCEPT_FIRST_HIT_AND_END_SEARCH query, shaders/path.slang:630-684: first hit ends the
  * walk, no back-face culling): out_occluded[n] = 1 when a surface lies within tmax. */
 vkb_status vkb_debug_occluded(vkb_scene* scene, uint32_t n, const float* rays7, uint32_t* out_occluded);
+/* Bounces of the context's last render that ran in one launch instead of the wavefront's
+ * kernels, summed over its waves. */
+uint32_t vkb_debug_path_bounces(vkb_ctx* ctx);
 
 #ifdef __cplusplus
 }

@@ -176,6 +176,7 @@ SIGNATURES = {
     "vkb_debug_trace": (C.c_int, [_P, C.c_uint32, C.POINTER(C.c_float), C.POINTER(C.c_float), C.POINTER(C.c_uint32),
                                   C.POINTER(C.c_float)]),
     "vkb_debug_occluded": (C.c_int, [_P, C.c_uint32, C.POINTER(C.c_float), C.POINTER(C.c_uint32)]),
+    "vkb_debug_path_bounces": (C.c_uint32, [_P]),
     "vkb_debug_tlas_stats": (C.c_int, [_P, C.POINTER(C.c_double), C.POINTER(C.c_uint32), C.POINTER(C.c_uint32)]),
     "vkb_display": (C.c_int, [_P, C.c_void_p, C.c_void_p, C.c_int, C.c_uint32, C.c_uint32, C.c_void_p, C.c_int]),
     "vkb_cache_create": (C.c_int, [_P, C.c_void_p, C.POINTER(_P)]),

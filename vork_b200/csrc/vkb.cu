@@ -393,6 +393,7 @@ struct vkb_ctx {
     size_t wave_capacity = 32u << 20;   // path slots per wave (autotuned); 7.4 GB of queues when full
     int trace_blocks_per_sm = 128;      // shade grid: at most SMs x this (autotuned)
     uint64_t launches = 0;
+    uint32_t path_bounces = 0;          // of the last render: bounces that k_paths took
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::vector<cudaEvent_t> kernel_events;
     std::vector<cudaEvent_t> cache_events;    // timed renders: around each radiance-cache query launch
@@ -916,7 +917,6 @@ void wave_kernels(vkb_ctx* c, const PathParams& p, uint32_t paths, uint32_t boun
             else launch_wave(early, k_paths<false, false>, grid, TRACE_BLOCK, st, p, first, bounces, most);
         }
         tot.launches++;
-        tot.trace_launches++;
     };
     if (whole) launch_paths(0u);
     for (uint32_t b = 0; b <= bounces && !whole; ++b) {
@@ -1257,6 +1257,7 @@ void run_engine(vkb_ctx* c, std::vector<EngineJob>& jobs, const WaveBuffers& w, 
     VKB_CUDA(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
     eng.collect(ms);
     tot = eng.tot;
+    c->path_bounces = tot.counters[15];
     for (size_t k = 0; k < jobs.size(); ++k) jobs[k] = eng.jobs[k];
 }
 
@@ -2089,6 +2090,7 @@ vkb_status vkb_debug_tlas_stats(vkb_scene* s, double* sah_cost, uint32_t* max_de
 }
 
 void* vkb_ctx_stream(vkb_ctx* c) { return c ? reinterpret_cast<void*>(c->stream) : nullptr; }
+uint32_t vkb_debug_path_bounces(vkb_ctx* c) { return c ? c->path_bounces : 0; }
 uint64_t vkb_scene_launch_count(vkb_scene* s) { return s ? s->launches : 0; }
 
 vkb_status vkb_debug_sampler_groups(vkb_ctx* c, uint32_t n, const uint32_t* px, const uint32_t* py, const uint32_t* index,

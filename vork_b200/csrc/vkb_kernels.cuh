@@ -506,7 +506,7 @@ struct PathParams {
     // [6] dropped paths, [7] path slots of this wave, [8] pixels of this wave's jobs
     // [9] radiance-cache records of this wave, [10] adaptive pixel-samples skipped,
     // [11], [12] rays the closest-hit and shadow traces have taken, [13] this bounce's hits,
-    // [14] k_paths has taken the wave's remaining bounces
+    // [14] k_paths has taken the wave's remaining bounces, [15] how many those were (all waves)
     uint32_t* counters;
     unsigned long long* work;  // instrumented traversal: closest nodes, tris, instances, blas nodes; shadow nodes, tris, blas nodes
     uint32_t* err;
@@ -1594,7 +1594,10 @@ __global__ void __launch_bounds__(TRACE_BLOCK, PATHS_BLOCKS) k_paths(const __gri
     const uint32_t n = p.counters[cur], lane = threadIdx.x & 31u;
     const uint32_t share = short_share(n, gridDim.x * (TRACE_BLOCK / 32u)), i = share_index(share);
     if (share == 0u || n > most) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) p.counters[14] = 1u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (n != 0u && p.counters[14] == 0u) p.counters[15] += bounces - first + 1u;
+        p.counters[14] = 1u;
+    }
     const Job& J = p.job0;
     bool alive = lane < share && i < n;
     uint32_t slot = 0, rays = 0, entries = 0;
