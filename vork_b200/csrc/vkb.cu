@@ -1486,7 +1486,11 @@ void build_blas_gpu(vkb_scene* s, uint32_t builder, cudaStream_t st) {
     VKB_CUDA(cudaStreamSynchronize(st));
     for (const MeshInfo& mi : s->mesh_info) {
         const uint32_t n = mi.num_triangles;
-        if (n == 0) continue;
+        if (n == 0) {   // its box may still be entered: its vertices have one
+            const Bvh4Node none = empty_node();
+            VKB_CUDA(cudaMemcpyAsync(s->blas4.p + mi.node_offset, &none, sizeof(none), cudaMemcpyHostToDevice, st));
+            continue;
+        }
         const uint32_t* idx = s->indices.p + mi.index_offset;
         k_tri_boxes<<<grid_for(n, 256, sms), 256, 0, st>>>(n, idx, s->vpos.p + mi.vertex_offset, s->tri_lo.p, s->tri_hi.p);
         const uint32_t* parents = s->scratch.node_parent.p;
@@ -1579,7 +1583,12 @@ vkb_status vkb_scene_create(vkb_ctx* ctx, const vkb_scene_desc* d, vkb_scene** o
                 const vkb_mesh& me = d->meshes[m];
                 uint32_t n = mi.num_triangles;
                 mi.node_offset = uint32_t(wide8 ? all_nodes8.size() : all_nodes.size());
-                if (n == 0) continue;
+                // A mesh without triangles may have vertices, and then a box that rays enter.
+                if (n == 0) {
+                    if (wide8) all_nodes8.push_back(Bvh8Node{});   // no slot in use
+                    else all_nodes.push_back(empty_node());
+                    continue;
+                }
                 std::vector<float> lo(3 * size_t(n)), hi(3 * size_t(n)), cen(3 * size_t(n));
                 for (uint32_t t = 0; t < n; ++t)
                     for (int a = 0; a < 3; ++a) {

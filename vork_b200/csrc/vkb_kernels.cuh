@@ -365,6 +365,12 @@ __device__ __host__ __forceinline__ void set_slot(Bvh4Node& q, int k, float lx, 
     reinterpret_cast<int*>(&q.child)[k] = ref;
     reinterpret_cast<int*>(&q.child2)[k] = ref;
 }
+// A node that every ray misses: the BLAS of a mesh without triangles.
+__host__ __forceinline__ Bvh4Node empty_node() {
+    Bvh4Node q;
+    for (int k = 0; k < 4; ++k) set_slot(q, k, INFINITY, -INFINITY, INFINITY, -INFINITY, INFINITY, -INFINITY, ~0);
+    return q;
+}
 // The slots of the 4-wide node for binary node b: each leaf child keeps its slot, each
 // internal child gives its own two children (internal references stay binary indices).
 __device__ __host__ __forceinline__ Bvh4Node collapse_node(const BvhNode* n2, const BvhNode& b) {
