@@ -700,7 +700,7 @@ __device__ __forceinline__ bool trace_any(const SceneView& sv, float4 o, float4 
 #define VKB_STACK_DECL_W(W8)                                                                             \
     __shared__ int stack_r_[SMEM_STACK * TRACE_BLOCK];                                                  \
     __shared__ float world_[WORLD_FLOATS * TRACE_BLOCK];                                                \
-    int stack_spill_[(W8) ? SPILL_STACK8 : (SPILL_STACK > 0 ? SPILL_STACK : 1)];                         \
+    int stack_spill_[(W8) ? SPILL_STACK8 : SPILL_STACK];                                                 \
     TraceStack stk{stack_r_ + threadIdx.x, stack_spill_, world_ + threadIdx.x};
 #define VKB_STACK_DECL VKB_STACK_DECL_W(false)
 // Lanes of a warp refill together once at most this many are still tracing.
