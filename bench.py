@@ -134,10 +134,10 @@ class ClockSampler:
 # fp32 corners), an instance entry 64 B (its TLAS leaf record: world->object rows and BLAS
 # references), and a ray 32 B of queue entry read plus a 24 B hit record written.
 NODE_BYTES, TRI_BYTES, INSTANCE_BYTES, RAY_BYTES = 80, 36, 64, 32 + 24
-# What the 4-wide FP32 node format actually stores and the kernel requests per visit:
-# 112 of its 128 bytes (6 face planes x 16 B + four child references), 48 B per stored
-# triangle (3 x float4), 20 B per hit record.
-STORED_NODE_BYTES, STORED_TRI_BYTES, STORED_RAY_BYTES = 112, 48, 32 + 20
+# What the 4-wide FP32 node format actually stores and the kernel requests per visit: its
+# whole 128 bytes, four 32-byte sectors (6 face planes x 16 B, the four child references
+# twice), 48 B per stored triangle (3 x float4), 20 B per hit record.
+STORED_NODE_BYTES, STORED_TRI_BYTES, STORED_RAY_BYTES = 128, 48, 32 + 20
 
 
 def roofline_bytes(stats: dict) -> float:

@@ -269,6 +269,8 @@ vkb_status vkb_close(vkb_ctx* ctx);
 /* Renderer::install + FrameRays::new (lib.rs:1322-1470; rt.rs:1098-1385): uploads the
  * descriptor (copied; the caller may free it on return) and builds every BLAS and the TLAS. */
 vkb_status vkb_scene_create(vkb_ctx* ctx, const vkb_scene_desc* desc, vkb_scene** out);
+/* The context keeps up to 256 MiB of the device buffers for later scenes, until it is
+ * closed or an allocation of this library runs out of memory. */
 vkb_status vkb_scene_destroy(vkb_scene* scene);
 
 /* rt::encode / rebuild_tlas (rt.rs:1387-1476): new object->world rows for every
@@ -334,7 +336,9 @@ vkb_status vkb_autotune(vkb_ctx* ctx, vkb_job* jobs, uint32_t njobs, vkb_tune_re
  * (crates/vork-cli/src/session.rs:1-60). */
 typedef struct vkb_server vkb_server;
 typedef struct vkb_server_config {
-    uint64_t memory_budget_bytes;  /* 0: unbounded */
+    uint64_t memory_budget_bytes;  /* 0: unbounded.  Scenes count as allocated (buffers kept from other
+                                      scenes may be up to a MiB larger each); a request that nothing runs
+                                      beside counts as what its scene asked for */
     uint32_t max_jobs;             /* admitted requests at once (job-table entries) */
     uint32_t flags;                /* VKB_PROFILE_* switches for every wave */
     uint64_t wave_capacity;        /* path slots per wave (0: the context's autotuned value) */
@@ -365,7 +369,7 @@ vkb_status vkb_server_destroy(vkb_server* server);
 typedef struct vkb_scene_info_t {
     uint64_t num_instances;
     uint64_t num_triangles;
-    uint64_t scene_bytes;      /* device bytes of meshes, BLAS, TLAS and instance records */
+    uint64_t scene_bytes;      /* device bytes of meshes, BLAS, TLAS and instance records, as allocated */
     uint64_t tlas_rebuilds;
     uint64_t tlas_refits;
     uint64_t motion_bytes;     /* changed object bytes accumulated since the last rebuild */

@@ -112,7 +112,7 @@ class Renderer:
         return images, {k: getattr(st, k) for k, _ in abi.VkbStats._fields_}
 
     def autotune(self, items) -> dict:
-        """Pick the wave capacity and trace grid for these jobs (vkb_autotune)."""
+        """Pick the wave capacity and shade grid for these jobs (vkb_autotune)."""
         n = len(items)
         jobs = (abi.VkbJob * max(1, n))()
         for k, (inst, prof) in enumerate(items):

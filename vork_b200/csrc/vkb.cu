@@ -391,7 +391,7 @@ struct vkb_ctx {
     DBuf<float4> accum, staging;        // per-render accumulators and host-output staging (all jobs of a call)
     DBuf<uint32_t> ids;                 // primary ids of the jobs that asked for them
     size_t wave_capacity = 32u << 20;   // path slots per wave (autotuned); 7.4 GB of queues when full
-    int trace_blocks_per_sm = 128;      // shade grid: at most SMs x this (autotuned)
+    int shade_blocks_per_sm = 128;      // shade grid: at most SMs x this (autotuned)
     uint64_t launches = 0;
     uint32_t path_bounces = 0;          // of the last render: bounces that k_paths took
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -844,7 +844,7 @@ struct WaveGrids {
         const uint32_t sms = uint32_t(c->sms);
         trace = int(std::max(1u, std::min((paths + 15u) / 16u, sms * VKB_TRACE_MIN_BLOCKS)));
         split = int(std::max(1u, std::min((paths + SPLIT_BLOCK * SPLIT_EACH - 1u) / (SPLIT_BLOCK * SPLIT_EACH), sms * 16u)));
-        shade = int(std::max(std::min((paths + 63u) / 64u, sms), std::min((paths + SHADE_BLOCK - 1u) / SHADE_BLOCK, sms * uint32_t(c->trace_blocks_per_sm))));
+        shade = int(std::max(std::min((paths + 63u) / 64u, sms), std::min((paths + SHADE_BLOCK - 1u) / SHADE_BLOCK, sms * uint32_t(c->shade_blocks_per_sm))));
     }
 };
 
@@ -1910,7 +1910,7 @@ vkb_status vkb_autotune(vkb_ctx* c, vkb_job* jobs, uint32_t njobs, vkb_tune_resu
     if (!c || !jobs || njobs == 0) return fail(VKB_INVALID_ARG, "null context or no jobs");
     return guarded([&] {
         VKB_CUDA(cudaSetDevice(c->device));
-        // Candidates: wave capacity (queue slots) x trace/shade blocks per SM, each timed on
+        // Candidates: wave capacity (queue slots) x most shade blocks per SM, each timed on
         // one sample of every job (same work for every candidate).
         const size_t caps[] = {size_t(2) << 20, size_t(4) << 20, size_t(8) << 20, size_t(16) << 20, size_t(32) << 20};
         const int grids[] = {32, 64, 128};
@@ -1928,13 +1928,13 @@ vkb_status vkb_autotune(vkb_ctx* c, vkb_job* jobs, uint32_t njobs, vkb_tune_resu
         }
         c->staging.alloc(1);
         size_t best_cap = c->wave_capacity;
-        int best_grid = c->trace_blocks_per_sm;
+        int best_grid = c->shade_blocks_per_sm;
         float best_ms = INFINITY;
         uint32_t tried = 0;
         for (size_t cap : caps)
             for (int g : grids) {
                 c->wave_capacity = std::max(cap, max_pix);
-                c->trace_blocks_per_sm = g;
+                c->shade_blocks_per_sm = g;
                 // Device outputs into the staging buffer region (results are discarded).
                 size_t total = 0;
                 for (uint32_t k = 0; k < njobs; ++k) total += size_t(in[k].first->camera.width) * in[k].first->camera.height;
@@ -1960,7 +1960,7 @@ vkb_status vkb_autotune(vkb_ctx* c, vkb_job* jobs, uint32_t njobs, vkb_tune_resu
                 if (tot.render_ms < best_ms) { best_ms = tot.render_ms; best_cap = c->wave_capacity; best_grid = g; }
             }
         c->wave_capacity = best_cap;
-        c->trace_blocks_per_sm = best_grid;
+        c->shade_blocks_per_sm = best_grid;
         if (out) {
             out->tried = tried;
             out->best_capacity = uint64_t(best_cap);

@@ -639,8 +639,8 @@ __device__ __forceinline__ uint32_t find_job(const PathParams& p, uint32_t x) {
 // A pixel's samples take neighbouring slots, and so do its later rays (every pass packs its
 // queue in order): the lanes of a warp then read mostly the same nodes and shade the same
 // surfaces.  With a pixel's samples an image apart, whole renders took 3-6% longer (1080p
-// 64 spp flock frame 375.8 vs 365.4 ms, 256x256 16 spp 1.99 vs 1.88 ms, preview batch 34.9 vs
-// 33.8 ms); tiles of 4 or 8 image rows under this order: equal or 1% slower.
+// 64 spp flock frame 375.8 vs 365.4 ms, 256x256 16 spp 1.99 vs 1.88 ms, a batch of 24 previews
+// (larger ones than the batch of k_split's figures) 34.9 vs 33.8 ms); tiles of 4 or 8 image rows under this order: equal or 1% slower.
 template <bool BATCH>
 __global__ void k_camera(PathParams p) {
     cudaGridDependencySynchronize();
@@ -753,7 +753,7 @@ __device__ __forceinline__ uint32_t share_index(uint32_t share) {
 //    warp's idle lanes together once at most VKB_TRACE_REFILL still trace (each lane as soon
 //    as it finishes is slower: that code then runs on single lanes).
 // 419 warp instructions per ray; the frame 483.0 -> 400.9 ms with the shadow rays done
-// the same way, 256x256 16 spp 2.72 -> 2.37 ms.
+// the same way (an earlier box: 583 -> 479 ms), 256x256 16 spp 2.72 -> 2.37 ms.
 template <bool COUNT, bool BATCH, bool W8 = false>
 __global__ void __launch_bounds__(TRACE_BLOCK, VKB_TRACE_MIN_BLOCKS) k_trace(PathParams p, int cur) {
     cudaGridDependencySynchronize();

@@ -15,8 +15,9 @@ namespace vkb_host {
 // Device buffers that scenes and calls of one context gave back, for the next ones: an
 // install takes some forty buffers and a display call three, and cudaMalloc / cudaFree (which
 // waits for the device) took most of a small scene's install (20,000 birds on the GPU
-// builders, first frame of 640x360: 14-25 ms from process to process, 4.3 ms with kept
-// buffers).  Bounded; a buffer comes back only when no work on any stream still uses it; what
+// builders, first frame of 640x360: 14-25 ms from process to process, 4.0-4.3 ms with kept
+// buffers; a 1080p display call 3.3 -> 2.2 ms in a process that makes it over and over, but
+// its time is pageable copies and varies between processes by more than that).  Bounded; a buffer comes back only when no work on any stream still uses it; what
 // is idle is freed when the context closes or when an allocation of this library runs out of
 // memory (device_alloc).
 template <class Api> class DevicePool {
